@@ -244,7 +244,9 @@ int rg_build_bvh(const float *tri_xyz, int32_t n_tris, rg_aabb_tree_node *out_no
  * contents byte-identical to rg_build_bvh's.  Synchronous on `stream`;
  * returns the node count; *ref_undefined (host, may be null) is set when a
  * range took a path the reference leaves undefined (see rg_build_bvh).
- * At most 4,194,304 triangles; coordinates must be finite.  No counterpart
+ * At most 4,194,304 triangles; coordinates must be finite.  The context keeps
+ * the workspace (about 170 bytes per triangle) for later calls until it is
+ * destroyed.  No counterpart
  * in the reference, which builds on the host (aabbTreeBuilder.cpp:52-214). */
 int rg_build_bvh_device(rg_context *ctx, const float *tri_xyz, int32_t n_tris, rg_aabb_tree_node *nodes,
                         rg_triangle *triangles, int32_t *ref_undefined, void *stream);

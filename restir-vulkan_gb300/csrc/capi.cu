@@ -108,6 +108,9 @@ struct rg_context {
     uint32_t vc_tag = 0;
     bool vc_on = true;        // rg_set_visibility_cache
     bool vc_dirty = true;     // clear before the next use (new scene, new buffers)
+    // workspace of rg_build_bvh_device (synchronous, so idle between calls)
+    unsigned char *tree_ws[2] = {nullptr, nullptr};
+    size_t tree_ws_bytes[2] = {0, 0};
 
     void release_scene() {
         proposal_release(proposal);
@@ -218,6 +221,8 @@ int rg_destroy(rg_context *ctx) {
     dev_free(ctx->mma_timeouts);
     dev_free(ctx->vc_buf[0]);
     dev_free(ctx->vc_buf[1]);
+    dev_free(ctx->tree_ws[0]);
+    dev_free(ctx->tree_ws[1]);
     delete ctx;
     return RG_OK;
 }
@@ -747,6 +752,17 @@ int rg_render_frame_host(rg_context *ctx, int32_t w, int32_t h, const uint8_t *a
 int rg_internal_fail(int code, const char *msg) { return fail(code, "%s", msg); }
 
 bool rg_internal_vcache_on(rg_context *ctx) { return ctx->vc_on; }
+
+int rg_internal_tree_workspace(rg_context *ctx, int slot, size_t bytes, void **out) {
+    if (bytes > ctx->tree_ws_bytes[slot]) {
+        dev_free(ctx->tree_ws[slot]);
+        ctx->tree_ws_bytes[slot] = 0;
+        RG_CUDA(dev_alloc(&ctx->tree_ws[slot], bytes), "tree builder workspace");
+        ctx->tree_ws_bytes[slot] = bytes;
+    }
+    *out = ctx->tree_ws[slot];
+    return RG_OK;
+}
 
 ProposalState **rg_internal_proposal(rg_context *ctx) {
     cudaSetDevice(ctx->device);

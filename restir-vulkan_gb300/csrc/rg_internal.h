@@ -204,9 +204,9 @@ int rg_internal_check_spatial_args(const rg_gbuffer *g, const void *in, const vo
 // device's primary context, which unloads the module holding the array).
 void noalloc_forget_device(int device);
 
-// gpu_bvh.cu: the reference tree built on the device (node count, or < 0).
-int gpu_build_bvh(const float *xyz, int n, rg_aabb_tree_node *nodes, rg_triangle *tris, int *undefined,
-                  cudaStream_t st);
+// Device workspace of the tree builder (two slots), kept in the context and
+// grown when a call needs more; freed with the context.
+int rg_internal_tree_workspace(rg_context *ctx, int slot, size_t bytes, void **out);
 
 // proposal.cu: the learned proposal attached to a context.
 struct ProposalState;
