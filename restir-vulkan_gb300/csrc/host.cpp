@@ -488,19 +488,45 @@ inline float pow2f(int eb) {
 // D(q) for biased exponent eb and base c
 inline float qdecode(int q, int eb, float c) { return fmaf(8388608.0f + (float)q, pow2f(eb), c); }
 
+// The walk's base of an axis: plane q lies at c + (2^15 + q) s in real
+// arithmetic, with c rounded down from the base above.
+inline float walk_base(int eb, float base) {
+    const double v = (double)base + (8388608.0 - 32768.0) * (double)pow2f(eb);
+    float c = (float)v;
+    while ((double)c > v) c = std::nextafter(c, -INFINITY);
+    return c;
+}
+inline double walk_plane(int q, int eb, float c) { return (double)c + (32768.0 + q) * (double)pow2f(eb); }
+
+// Code q bounds lo from below (hi from above): decoded, and as the walk's
+// plane with 1/16 code to spare (see trace_pool.cuh for what that covers).
+inline bool code_below(int q, int eb, float base, float c, float lo) {
+    return qdecode(q, eb, base) <= lo && walk_plane(q, eb, c) <= (double)lo - 0.0625 * (double)pow2f(eb);
+}
+inline bool code_above(int q, int eb, float base, float c, float hi) {
+    return qdecode(q, eb, base) >= hi && walk_plane(q, eb, c) >= (double)hi + 0.0625 * (double)pow2f(eb);
+}
+
 // Base and biased exponent of one axis of a node with bounds [lo, hi]; false
-// when no exponent up to 246 (255 * s finite) reaches hi.
+// when no exponent up to 246 (255 * s finite) reaches hi.  A flat axis starts
+// at the exponent whose 255 codes span one unit in the last place of lo.
 bool quant_axis(float lo, float hi, float &c, int &eb) {
     const double ext = (double)hi - (double)lo;
     eb = 1;
     if (ext > 0.0) eb = std::max(1, std::min(246, (int)std::ceil(std::log2(ext / 254.0)) + 127));
+    int lo_exp = 0;
+    std::frexp(std::max(std::fabs(lo), std::fabs(hi)), &lo_exp);
+    eb = std::max(eb, std::min(246, lo_exp - 1 - 23 - 8 + 127));
     for (; eb <= 246; ++eb) {
         const float s = pow2f(eb);
         float cc = (float)((double)lo - std::ldexp(1.0, eb - 127 + 23));
         while (fmaf(8388608.0f, s, cc) > lo) cc = std::nextafter(cc, -INFINITY);
         while (fmaf(8388608.0f, s, std::nextafter(cc, INFINITY)) <= lo) cc = std::nextafter(cc, INFINITY);
-        const float top = qdecode(255, eb, cc);
-        if (std::isfinite(cc) && std::isfinite(top) && top >= hi) {
+        if (!std::isfinite(cc) || !std::isfinite(qdecode(255, eb, cc))) continue;
+        // a step lower where the walk's plane of code 0 needs it
+        for (int k = 0; k < 2 && !code_below(0, eb, cc, walk_base(eb, cc), lo); ++k) cc = std::nextafter(cc, -INFINITY);
+        const float w = walk_base(eb, cc);
+        if (code_below(0, eb, cc, w, lo) && code_above(255, eb, cc, w, hi)) {
             c = cc;
             return true;
         }
@@ -541,13 +567,14 @@ struct QuantBuilder {
             for (int a = 0; a < 3; ++a) {
                 // start from the real-valued estimate, then step to the exact codes
                 const double s = std::ldexp(1.0, eb[a] - 127), o = (double)base[a] + 8388608.0 * s;
+                const float wb = walk_base(eb[a], base[a]);
                 int ql = (int)std::max(0.0, std::min(255.0, std::floor(((double)c.lo[a] - o) / s)));
                 int qh = (int)std::max(0.0, std::min(255.0, std::ceil(((double)c.hi[a] - o) / s)));
-                while (ql > 0 && qdecode(ql, eb[a], base[a]) > c.lo[a]) --ql;
-                while (ql < 255 && qdecode(ql + 1, eb[a], base[a]) <= c.lo[a]) ++ql;
-                while (qh < 255 && qdecode(qh, eb[a], base[a]) < c.hi[a]) ++qh;
-                while (qh > 0 && qdecode(qh - 1, eb[a], base[a]) >= c.hi[a]) --qh;
-                if (!(qdecode(ql, eb[a], base[a]) <= c.lo[a]) || !(qdecode(qh, eb[a], base[a]) >= c.hi[a])) ok = false;
+                while (ql > 0 && !code_below(ql, eb[a], base[a], wb, c.lo[a])) --ql;
+                while (ql < 255 && code_below(ql + 1, eb[a], base[a], wb, c.lo[a])) ++ql;
+                while (qh < 255 && !code_above(qh, eb[a], base[a], wb, c.hi[a])) ++qh;
+                while (qh > 0 && code_above(qh - 1, eb[a], base[a], wb, c.hi[a])) --qh;
+                if (!code_below(ql, eb[a], base[a], wb, c.lo[a]) || !code_above(qh, eb[a], base[a], wb, c.hi[a])) ok = false;
                 w[4 + 2 * a] |= (uint32_t)ql << (8 * k);
                 w[5 + 2 * a] |= (uint32_t)qh << (8 * k);
             }
@@ -603,6 +630,53 @@ int32_t host_pack_quant(const rg_aabb_tree_node *src, int32_t n, const float *tr
     if (wide_depth) *wide_depth = b.max_depth;
     if (!b.ok) return -1;
     return (int32_t)(nodes.size() / 16);
+}
+
+// The packed nodes as the device walks them (QNode): bases for planes at
+// c + (2^15 + q) s, the scale of z with the slot masks in its low bits, inner
+// children in the first slots, a node's inner children consecutive (each
+// child's own children follow its group, first child first) and its leaf
+// records too, so a node holds two links.  Empty when a base or scale is
+// beyond 2^40, where the walk's products might overflow.
+std::vector<uint32_t> host_walk_nodes(const std::vector<uint32_t> &nodes) {
+    const float lim = 1099511627776.0f;
+    std::vector<uint32_t> out(nodes.size());
+    struct Item { uint32_t from, to; };
+    std::vector<Item> todo{{0u, 0u}};
+    uint32_t used = 1;
+    while (!todo.empty()) {
+        const Item it = todo.back();
+        todo.pop_back();
+        const uint32_t *w = &nodes[16 * (size_t)it.from];
+        uint32_t *d = &out[16 * (size_t)it.to];
+        const uint32_t leaf = (w[3] >> 24) & 15u, inner = w[3] >> 28;
+        int eb[3];
+        for (int a = 0; a < 3; ++a) {
+            eb[a] = (int)((w[3] >> (8 * a)) & 255u);
+            float base;
+            memcpy(&base, &w[a], 4);
+            const float c = walk_base(eb[a], base);
+            if (!(std::fabs(c) <= lim) || !(pow2f(eb[a]) <= lim)) return {};
+            memcpy(&d[a], &c, 4);
+        }
+        int slot_of[4], ni = 0, at = 0;  // packed slot of each slot here
+        for (int k = 0; k < 4; ++k)
+            if (inner >> k & 1u) slot_of[at++] = k;
+        ni = at;
+        for (int k = 0; k < 4; ++k)
+            if (leaf >> k & 1u) slot_of[at++] = k;
+        const uint32_t n_leaf = (uint32_t)(at - ni);
+        d[3] = ((uint32_t)eb[2] << 23) | (((1u << n_leaf) - 1u) << ni) | (((1u << ni) - 1u) << 4);
+        for (int q = 4; q < 10; ++q)
+            for (int k = 0; k < 4; ++k) d[q] |= ((w[q] >> (8 * slot_of[k < at ? k : at - 1])) & 255u) << (8 * k);
+        d[10] = w[10];
+        d[11] = w[11];
+        d[12] = used;
+        d[13] = n_leaf ? ~w[12 + slot_of[ni]] - (uint32_t)ni : 0u;  // its leaves were packed together
+        for (int k = ni - 1; k >= 0; --k) todo.push_back({w[12 + slot_of[k]], used + (uint32_t)k});
+        used += (uint32_t)ni;
+    }
+    return out;
 }
 
 // True when a child box coordinate of some node is NaN (e.g. a tree built

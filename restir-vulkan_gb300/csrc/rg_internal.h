@@ -45,16 +45,18 @@ struct WNode {
 };
 constexpr int32_t kWideNoChild = INT32_MIN;
 
-// QNode 64 B: the quantized 4-wide copy (host_pack_quant).  Per axis a base
-// c and a power of two s (biased exponent bytes in base.w); child k's bounds
-// are byte k of the axis' lower and upper code words, code q decoding to
-// RN((2^23 + q) * s + c), a box containing the child's exact box.  Links:
-// >= 0 node, < 0 leaf record ~r, kWideNoChild = empty.
+// QNode 64 B: the quantized 4-wide copy as the walk reads it
+// (host_walk_nodes).  Per axis a base c and a power of two s; child k's bounds
+// are byte k of the axis' lower and upper code words, code q standing for the
+// plane c + (2^15 + q) s, outside the child's exact box.  Inner children take
+// the first slots and are consecutive nodes, leaf children the next slots and
+// are consecutive leaf records.
 struct QNode {
-    float4 base; // c.xyz, exponent bytes (x, y, z) and slot masks (leaf bits 0-3, inner bits 4-7)
+    float4 base; // c.xyz; s of z, whose low bits are zero, with the slot masks in them (leaf
+                 // bits 0-3, inner bits 4-7)
     uint4 qxy;   // lo x, hi x, lo y, hi y (byte k: child k)
     uint4 qz;    // lo z, hi z, s of x, s of y (float bits)
-    int4 d;      // links of children 0..3
+    int4 d;      // first inner child's node, first leaf record - number of inner children, 0, 0
 };
 // QLeaf 64 B: a leaf of the quantized copy, the triangle's exact box from
 // the reference's tree and the triangle in GTri form.

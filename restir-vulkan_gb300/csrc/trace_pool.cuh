@@ -527,84 +527,87 @@ __device__ void trace_wide_loop(const DevScene &s, Fetch fetch, int n, int *next
     }
 }
 
-// Codes sel0, sel1 (byte selectors) of a word decoded as a packed pair:
-// D(q) = RN((2^23 + q) * s + c), one FMA on the float whose bits are
-// 0x4B000000 | q.
-__device__ __forceinline__ float2 qdecode2(unsigned w, unsigned sel0, unsigned sel1, float2 sc, float2 base) {
-    const float2 f = make_float2(__uint_as_float(__byte_perm(w, 0x4B000000u, sel0)),
-                                 __uint_as_float(__byte_perm(w, 0x4B000000u, sel1)));
-    return __ffma2_rn(f, sc, base);
+// 32 bytes through the read-only path as one 256-bit load (32-byte aligned).
+// Lanes of a warp read different nodes, so a load costs the L1 one data-pipe
+// cycle per lane whatever its width up to 32 bytes; with four 128-bit loads a
+// node that pipe was the walk's limit (69 % busy on average).
+__device__ __forceinline__ void ldg256(const void *p, float4 &a, float4 &b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+__device__ __forceinline__ uint4 as_uint4(float4 v) {
+    return make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
 }
 
-// Per-ray and per-node operands of the quantized box tests.  Each axis' near
-// and far code words are picked by the sign of the ray's direction (near =
-// lower bounds where it is positive), so the slab distances come out ordered:
-// t(near) <= t(far), because b - o and the product with 1/d round
-// monotonically; they equal the min and max of the two distances.
-struct QAxes {
-    unsigned nx, fx, ny, fy, nz, fz;  // near / far code words
-};
-__device__ __forceinline__ QAxes qaxes(f3 inv, const uint4 &qa, const uint4 &qb) {
-    QAxes a;
+// ---- the quantized walk's box test
+// Child k's plane with code q lies at P = c + (2^15 + q) s (real arithmetic;
+// c the node's base, s its power-of-two scale on the axis).  With f = 2^15 + q
+// (a float whose second byte is q: one byte permute), its distance along the
+// ray is one FMA,
+//   t = RN(f A + B),  A = s inv,  B = RN(RN(c - o) inv -+ K),  K = 2^-18,
+// where near planes take B with -K and far planes with +K.  Only a sure miss
+// may drop a child, so t has to bound the reference's t_ref = RN(RN(b - o)/d)
+// of the exact bound b, from below for near planes and from above for far
+// ones.  With u = 2^-24, C = (c - o)/d, F = f s/|d| <= 2^15.02 |A| and tau =
+// (P - o)/d, the roundings (c - o, inv, the product, the FMA) add up to at
+// most u (4 |tau| + 4 F + 2 K), that is 2^-22 |tau| + 2^-6.98 |A| + 2^-41.
+// The host places every plane at least s/16 outside b (host.cpp,
+// code_below / code_above), which pays for the second term, and K for the
+// others while |tau| <= 4: there near t < t_ref < far t.  Beyond, tau < -4 or
+// tau > 4 has the same sign and side of 1 as t_ref, and only the signs and
+// sides matter: a child is kept when
+//   max(0, near t's) < min(1, far t's),
+// which a reference hit (entry < 1, exit > 0, exit >= entry) implies.  The
+// clamps are the saturating form of the x axis' FMAs.  Magnitudes stay finite:
+// bases and scales are at most 2^40 (checked at upload), and the rays that
+// take this walk have |o| <= 2^40 and |d| in [2^-60, 2^60] (ray_fits); A or a
+// product that underflows is far below K.
+// Each axis' near and far code words are picked by the ray's direction sign.
+// Against decoding each plane, subtracting o and multiplying by inv (three
+// packed operations a plane instead of one), 1080p frames with 1.05M
+// triangles: see DESIGN's table for the measured passes.
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+    float y;
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
+__device__ __forceinline__ float code_float(unsigned w, unsigned k) {
+    return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7604u | (k << 4)));
+}
+constexpr float kWalkK = 3.814697265625e-6f;  // 2^-18
+
+// Slot bits of the children that are not surely missed.
+__device__ __forceinline__ unsigned qlive(f3 o, f3 inv, const float4 &base, const uint4 &qa, const uint4 &qb) {
     const bool sx = inv.x < 0.0f, sy = inv.y < 0.0f, sz = inv.z < 0.0f;
-    a.nx = sx ? qa.y : qa.x; a.fx = sx ? qa.x : qa.y;
-    a.ny = sy ? qa.w : qa.z; a.fy = sy ? qa.z : qa.w;
-    a.nz = sz ? qb.y : qb.x; a.fz = sz ? qb.x : qb.y;
-    return a;
+    const unsigned nx = sx ? qa.y : qa.x, fx = sx ? qa.x : qa.y;
+    const unsigned ny = sy ? qa.w : qa.z, fy = sy ? qa.z : qa.w;
+    const unsigned nz = sz ? qb.y : qb.x, fz = sz ? qb.x : qb.y;
+    const float ax = __uint_as_float(qb.z) * inv.x, ay = __uint_as_float(qb.w) * inv.y,
+                az = __uint_as_float(__float_as_uint(base.w) & 0x7f800000u) * inv.z;
+    const float cx = base.x - o.x, cy = base.y - o.y, cz = base.z - o.z;
+    const float bnx = __fmaf_rn(cx, inv.x, -kWalkK), bfx = __fmaf_rn(cx, inv.x, kWalkK);
+    const float2 by = make_float2(__fmaf_rn(cy, inv.y, -kWalkK), __fmaf_rn(cy, inv.y, kWalkK));
+    const float2 bz = make_float2(__fmaf_rn(cz, inv.z, -kWalkK), __fmaf_rn(cz, inv.z, kWalkK));
+    const float2 ay2 = make_float2(ay, ay), az2 = make_float2(az, az);
+    unsigned live = 0u;
+#pragma unroll
+    for (unsigned k = 0; k < 4; ++k) {
+        const float tnx = fma_sat(code_float(nx, k), ax, bnx), tfx = fma_sat(code_float(fx, k), ax, bfx);
+        const float2 ty = __ffma2_rn(make_float2(code_float(ny, k), code_float(fy, k)), ay2, by);
+        const float2 tz = __ffma2_rn(make_float2(code_float(nz, k), code_float(fz, k)), az2, bz);
+        if (max3f(tnx, ty.x, tz.x) < min3f(tfx, ty.y, tz.y)) live |= 1u << k;
+    }
+    return live;
 }
-
-// The sure-miss part of the filtered decision with a constant difference
-// margin: where rmin~ <= 1 + E and rmax~ >= -T, a difference below -SS
-// needs rmax~ < rmin~, so both lie in [-T, 1 + E] and E (|rmin~| + |rmax~|)
-// + T < 2^-17 = SS; the test is therefore never looser than
-// filtered_decision's.
-__device__ __forceinline__ bool filtered_miss(float rmin, float rmax) {
-    constexpr float kEps = 1.9073486328125e-6f;     // 2^-19
-    constexpr float kTiny = 8.0779356694631609e-28f; // 2^-90
-    constexpr float kSS = 7.62939453125e-6f;         // 2^-17
-    return rmin > 1.0f + kEps || rmax < -kTiny || rmax - rmin < -kSS;
-}
-
-// RG_QMISS_SIGN: the quantized walk's sure-miss test as packed differences
-// and the sign of their minimum (moves compares from the ALU pipe to the FMA
-// pipe; 5.88 -> 5.80 ms per 1080p unbiased pass, same decisions).
-#ifndef RG_QMISS_SIGN
-#define RG_QMISS_SIGN 1
-#endif
-
-// Children 2p, 2p+1 of a quantized node: bit 0 / bit 1 set when the filtered
-// test does not surely miss their decoded boxes.
-__device__ __forceinline__ unsigned qpair_live(f3 o, f3 inv, const float4 &base, const QAxes &w, float2 sx,
-                                               float2 sy, float2 sz, int p) {
-    const unsigned s0 = 0x7440u + 2u * (unsigned)p, s1 = s0 + 1u;
-    const float2 cx = make_float2(base.x, base.x), cy = make_float2(base.y, base.y), cz = make_float2(base.z, base.z);
-    const float2 nox = make_float2(-o.x, -o.x), noy = make_float2(-o.y, -o.y), noz = make_float2(-o.z, -o.z);
-    const float2 ix = make_float2(inv.x, inv.x), iy = make_float2(inv.y, inv.y), iz = make_float2(inv.z, inv.z);
-    const float2 tnx = __fmul2_rn(__fadd2_rn(qdecode2(w.nx, s0, s1, sx, cx), nox), ix);
-    const float2 tfx = __fmul2_rn(__fadd2_rn(qdecode2(w.fx, s0, s1, sx, cx), nox), ix);
-    const float2 tny = __fmul2_rn(__fadd2_rn(qdecode2(w.ny, s0, s1, sy, cy), noy), iy);
-    const float2 tfy = __fmul2_rn(__fadd2_rn(qdecode2(w.fy, s0, s1, sy, cy), noy), iy);
-    const float2 tnz = __fmul2_rn(__fadd2_rn(qdecode2(w.nz, s0, s1, sz, cz), noz), iz);
-    const float2 tfz = __fmul2_rn(__fadd2_rn(qdecode2(w.fz, s0, s1, sz, cz), noz), iz);
-#if RG_QMISS_SIGN
-    // filtered_miss of both children as signs: RN(1 + E - rmin) < 0 iff
-    // rmin > 1 + E, RN(rmax + T) < 0 iff rmax < -T, RN(RN(rmax - rmin) + SS)
-    // < 0 iff RN(rmax - rmin) < -SS (no result is -0: each adds a nonzero
-    // constant; a NaN difference of two infinities is dropped by the minimum,
-    // as its comparison is false)
-    const float2 rmin = make_float2(max3f(tnx.x, tny.x, tnz.x), max3f(tnx.y, tny.y, tnz.y));
-    const float2 rmax = make_float2(min3f(tfx.x, tfy.x, tfz.x), min3f(tfx.y, tfy.y, tfz.y));
-    const float2 m1 = make_float2(-1.0f, -1.0f);
-    const float2 a = __ffma2_rn(rmin, m1, make_float2(1.0000019073486328125f, 1.0000019073486328125f));
-    const float2 b = __fadd2_rn(rmax, make_float2(8.0779356694631609e-28f, 8.0779356694631609e-28f));
-    const float2 c = __fadd2_rn(__ffma2_rn(rmin, m1, rmax), make_float2(7.62939453125e-6f, 7.62939453125e-6f));
-    const unsigned ml = __float_as_uint(min3f(a.x, b.x, c.x)) >> 31, mr = __float_as_uint(min3f(a.y, b.y, c.y)) >> 31;
-    return (ml ^ 1u) | ((mr ^ 1u) << 1);
-#else
-    const bool ml = filtered_miss(max3f(tnx.x, tny.x, tnz.x), min3f(tfx.x, tfy.x, tfz.x));
-    const bool mr = filtered_miss(max3f(tnx.y, tny.y, tnz.y), min3f(tfx.y, tfy.y, tfz.y));
-    return (ml ? 0u : 1u) | (mr ? 0u : 2u);
-#endif
+// Whether the ray may take the quantized walk (finite products above); the
+// others walk the reference's tree exactly.
+__device__ __forceinline__ bool ray_fits(f3 o, f3 d) {
+    constexpr float kLo = 8.67361737988403547e-19f, kHi = 1.152921504606846976e18f;  // 2^-60, 2^60
+    constexpr float kPos = 1099511627776.0f;                                         // 2^40
+    const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
+    return fminf(fminf(ax, ay), az) >= kLo && max3f(ax, ay, az) <= kHi &&
+           max3f(fabsf(o.x), fabsf(o.y), fabsf(o.z)) <= kPos;
 }
 
 // The exact slab test of a leaf record's box (undecided filtered tests only).
@@ -615,7 +618,9 @@ __device__ __noinline__ bool leaf_box_exact(f3 o, f3 d, float4 a, float4 b) {
 // A leaf of the quantized copy: the reference's slab test of the triangle's
 // exact box (filtered, exact where undecided), then its triangle test.
 __device__ __forceinline__ bool qleaf_hit(const QLeaf *lp, f3 o, f3 d, f3 inv) {
-    const float4 a = __ldg(&lp->a), b = __ldg(&lp->b), c = __ldg(&lp->c), e = __ldg(&lp->d);
+    float4 a, b, c, e;
+    ldg256(&lp->a, a, b);
+    ldg256(&lp->c, c, e);
     const float2 tx = __fmul2_rn(__fadd2_rn(make_float2(a.x, a.w), make_float2(-o.x, -o.x)), make_float2(inv.x, inv.x));
     const float2 ty = __fmul2_rn(__fadd2_rn(make_float2(a.y, b.x), make_float2(-o.y, -o.y)), make_float2(inv.y, inv.y));
     const float2 tz = __fmul2_rn(__fadd2_rn(make_float2(a.z, b.y), make_float2(-o.z, -o.z)), make_float2(inv.z, inv.z));
@@ -627,73 +632,70 @@ __device__ __forceinline__ bool qleaf_hit(const QLeaf *lp, f3 o, f3 d, f3 inv) {
     return hit && rgm::ray_tri(mk(b.z, b.w, c.x), mk(c.y, c.z, c.w), mk(e.x, e.y, e.z), o, d);
 }
 
-// RG_LEAF_SLOTS: parked leaf sets a lane may hold in the quantized walk (1
-// or 2).  With two, a lane that parks a node's leaves keeps walking until it
-// parks a second set, so fewer lanes sit idle in the walk phase and the leaf
-// phase tests more lanes at once.
-#ifndef RG_LEAF_SLOTS
-#define RG_LEAF_SLOTS 2
-#endif
 // Node visits per walking lane per pass through the quantized walk's warp
 // loop (with two leaf slots lanes stop less often: 8, 12, 16, 24, 32 steps
 // give 5.60, 5.49, 5.44, 5.63, 5.99 ms per 1080p unbiased pass).
 #ifndef RG_QWALK_STEPS
 #define RG_QWALK_STEPS 16
 #endif
-
-
-// RG_LEAF_COMPACT: the leaf phase lists the leaves every holding lane has
-// parked and tests them with all lanes of the warp (1 KB of shared memory per
-// warp), instead of each lane looping over its own.
-#ifndef RG_LEAF_COMPACT
-#define RG_LEAF_COMPACT 1
+// RG_QSTACK_SHARED: the quantized walk's stack in shared memory.
+#ifndef RG_QSTACK_SHARED
+#define RG_QSTACK_SHARED 0
 #endif
+
 #ifndef RG_UNBIASED_BT
 #define RG_UNBIASED_BT 128
 #endif
 constexpr int kLeafQueueWarps = (RG_UNBIASED_BT > 128 ? RG_UNBIASED_BT : 128) / 32;  // the largest pool block
 
-// The parked leaves of one node ((node << 4) | mask of its leaf slots): the
-// exact box gate and the triangle test of each until one hits.
-__device__ __forceinline__ bool qparked_hit(const DevScene &s, unsigned e, f3 o, f3 d, f3 inv, TraceStats &ts) {
-    const int4 ch = __ldg(&s.qnodes[e >> 4].d);
-    bool hit = false;
-    for (unsigned m = e & 15u; m != 0u && !hit; m &= m - 1u) {
-        const int k = __ffs(m) - 1;
-        const int link = k == 0 ? ch.x : k == 1 ? ch.y : k == 2 ? ch.z : ch.w;
-        hit = qleaf_hit(s.qleaves + ~link, o, d, inv);
-        ++ts.tri_tests;
-    }
-    return hit;
-}
+// Entries of the quantized walk's stack: at most one per level of the copy,
+// and the upload takes copies of up to RG_MAX_TREE_DEPTH / 3 levels.
+constexpr int kQStack = RG_MAX_TREE_DEPTH / 3;
 
 // The loop over the quantized 4-wide copy (DevScene::qnodes): a node visit
-// decodes its four child boxes and drops those the filtered test surely
-// misses (a decoded box contains the exact one, so the reference's test
-// misses the exact box too); the rest are walked (inner) or parked (leaves).
-// A parked leaf is tested with its exact box, then its triangle, so a
-// triangle is tested exactly when the reference's test passes its box,
-// which on a nested tree implies its whole box path passes, as in the
-// reference's walk.  Stack and order as in trace_wide_loop.
+// drops the children whose box the ray surely misses (qlive; a box stored in
+// the node contains the exact one, so the reference's test misses the exact
+// box too); the rest are walked (inner) or parked (leaves).  A parked leaf is
+// tested with its exact box, then its triangle, so a triangle is tested
+// exactly when the reference's test passes its box, which on a nested tree
+// implies its whole box path passes, as in the reference's walk.
+//
+// A node's inner children are consecutive nodes, its leaves consecutive leaf
+// records, so what is left to walk of a node is (first child, slot mask) in
+// one word: a visit pushes at most one word, and nothing while the node it
+// came from has no child left.  Every node is visited at most once.
+//
+// Each lane may hold two parked leaf sets (record of slot 0 << 4 | slot mask,
+// the record modulo 2^27), so it
+// keeps walking past its first leaves; the leaf phase lists the leaves every
+// holding lane has parked (1 KB of shared memory per warp) and tests them with
+// all lanes of the warp.
 template <typename Fetch, typename Endpoint, typename Emit>
-__device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *next, TraceStats &ts, Endpoint endpoint,
-                                 Emit emit) {
+__device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *next, int *stack, TraceStats &ts,
+                                 Endpoint endpoint, Emit emit) {
     constexpr unsigned kFull = 0xffffffffu;
-#if RG_LEAF_COMPACT
     __shared__ uint32_t s_leafq[kLeafQueueWarps][32 * 8];  // per warp: up to 8 parked leaves per lane
+    const int tid = threadIdx.x + threadIdx.y * blockDim.x;
+    const int lane = tid & 31;
+#if RG_QSTACK_SHARED
+    int *my_stack = stack + tid;
+    const int stride = blockDim.x * blockDim.y;
+#else
+    int my_stack[kQStack];
+    constexpr int stride = 1;
+    (void)stack;
 #endif
-    int my_stack[RG_MAX_TREE_DEPTH + 1];
-    int cur = -1;          // pool index of this lane's segment, -1: none
+    bool busy = false;     // this lane has a segment
     bool retired = false;  // the pool has no segment left for this lane
-    int owner = 0, node = 0, sp = 0, visits = 0;
-    unsigned park0 = 0u, park1 = 0u;  // parked leaves, (node << 4) | leaf slot mask; 0: none
-    bool walked = false;   // tree walk finished, only parked leaves remain
+    int owner = 0, sp = 0, visits = 0;
+    unsigned gbase = 0u, gmask = 0u;  // nodes to walk: gbase + each set bit (0-3)
+    unsigned park0 = 0u, park1 = 0u;  // parked leaf sets, 0: none
     f3 o = mk(0.f, 0.f, 0.f), d = o, inv = o;
     while (true) {
         // 1. refill idle lanes, several at a time
-        const bool idle = !retired && cur < 0;
+        const bool idle = !retired && !busy;
         const unsigned m_idle = __ballot_sync(kFull, idle);
-        const unsigned m_busy = __ballot_sync(kFull, cur >= 0);
+        const unsigned m_busy = __ballot_sync(kFull, busy);
         if (m_idle != 0u && (__popc(m_idle) >= RG_FETCH_MIN || m_busy == 0u)) {
             if (idle) {
                 ts.visits += (unsigned)visits;  // the finished segment's node visits
@@ -706,13 +708,12 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
                     ++ts.skipped;
                 } else {
                     rgm::shadow_segment(p1, endpoint(owner), o, d);
-                    if (ray_inverse(d, inv)) {
-                        cur = k;
-                        node = 0;
+                    if (ray_inverse(d, inv) && ray_fits(o, d)) {
+                        busy = true;
+                        gbase = 0u;
+                        gmask = 1u;  // the root
                         sp = 0;
-                        visits = 0;
                         park0 = park1 = 0u;
-                        walked = false;
                     } else {
                         emit(owner, trace_exact_binary(s, o, d, ts));
                     }
@@ -721,19 +722,17 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
         }
         if (__all_sync(kFull, retired)) break;
         // 2. parked leaves, once enough lanes cannot walk on (walk ended or
-        //    every slot taken) or none can; every lane holding some tests them
-        const bool blocked = cur >= 0 && (walked || (RG_LEAF_SLOTS == 1 ? park0 : park1) != 0u);
+        //    both slots taken) or none can; every lane holding some tests them
+        const bool blocked = busy && (gmask == 0u || park1 != 0u);
         const unsigned m_block = __ballot_sync(kFull, blocked);
-        const unsigned m_walk = __ballot_sync(kFull, cur >= 0 && !blocked);
+        const unsigned m_walk = __ballot_sync(kFull, busy && !blocked);
         if (m_block != 0u && (__popc(m_block) >= RG_LEAF_MIN || m_walk == 0u)) {
-#if RG_LEAF_COMPACT
             // the holders' leaves go to the warp's queue ((lane << 27) |
             // record), and every lane tests queued leaves, a chunk of 32 at a
             // time, with the owning lane's ray taken by shuffles; a ray's
             // remaining leaves are skipped once one of its leaves hits
-            const int lane = (threadIdx.x + threadIdx.y * blockDim.x) & 31;
-            uint32_t *q = s_leafq[(threadIdx.x + threadIdx.y * blockDim.x) >> 5];
-            const bool holder = cur >= 0 && park0 != 0u;
+            uint32_t *q = s_leafq[tid >> 5];
+            const bool holder = busy && park0 != 0u;
             const int cnt = holder ? __popc(park0 & 15u) + __popc(park1 & 15u) : 0;
             int incl = cnt;
 #pragma unroll
@@ -747,13 +746,8 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
 #pragma unroll
                 for (int slot = 0; slot < 2; ++slot) {
                     const unsigned e = slot == 0 ? park0 : park1;
-                    if (e == 0u) continue;
-                    const int4 ch = __ldg(&s.qnodes[e >> 4].d);
-                    for (unsigned m = e & 15u; m != 0u; m &= m - 1u) {
-                        const int k = __ffs(m) - 1;
-                        const int link = k == 0 ? ch.x : k == 1 ? ch.y : k == 2 ? ch.z : ch.w;
-                        q[at++] = ((unsigned)lane << 27) | (unsigned)(~link);
-                    }
+                    for (unsigned m = e & 15u; m != 0u; m &= m - 1u)
+                        q[at++] = ((unsigned)lane << 27) | (((e >> 4) + (unsigned)(__ffs(m) - 1)) & 0x7ffffffu);
                 }
             }
             __syncwarp();
@@ -777,22 +771,12 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
             if (holder) {
                 const bool hit = ((hits >> lane) & 1u) != 0u;
                 park0 = park1 = 0u;
-                if (hit || walked) {
+                if (hit || gmask == 0u) {
                     emit(owner, hit);
-                    cur = -1;
+                    busy = false;
+                    gmask = 0u;
                 }
             }
-#else
-            if (cur >= 0 && park0 != 0u) {
-                bool hit = qparked_hit(s, park0, o, d, inv, ts);
-                if (!hit && park1 != 0u) hit = qparked_hit(s, park1, o, d, inv, ts);
-                park0 = park1 = 0u;
-                if (hit || walked) {
-                    emit(owner, hit);
-                    cur = -1;
-                }
-            }
-#endif
             continue;
         }
         // 3. up to RG_QWALK_STEPS nodes per walking lane.  The copy is built on
@@ -800,50 +784,47 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
         //    upload), so a walk visits each node at most once; the visit count
         //    is checked here, once per pass through this loop rather than per
         //    visit (at most RG_QWALK_STEPS visits past the limit)
-        if (cur >= 0 && !walked && visits > s.n_qnodes) {
+        if (gmask != 0u && visits > s.n_qnodes) {
             ts.err = true;
             emit(owner, false);
-            cur = -1;
+            busy = false;
+            gmask = 0u;
             park0 = park1 = 0u;
         }
 #pragma unroll 1
-        for (int step = 0; step < RG_QWALK_STEPS && cur >= 0 && !walked &&
-                           (RG_LEAF_SLOTS == 1 ? park0 : park1) == 0u;
-             ++step) {
+        for (int step = 0; step < RG_QWALK_STEPS && gmask != 0u && park1 == 0u; ++step) {
             ++visits;
-            const QNode *np = s.qnodes + node;
-            const float4 base = __ldg(&np->base);
-            const uint4 qa = __ldg(&np->qxy), qb = __ldg(&np->qz);
-            const int4 ch = __ldg(&np->d);
-            const unsigned eb = __float_as_uint(base.w);
-            const float ex = __uint_as_float(qb.z), ey = __uint_as_float(qb.w),
-                        ez = __uint_as_float(((eb >> 16) & 0xffu) << 23);
-            const float2 sx = make_float2(ex, ex), sy = make_float2(ey, ey), sz = make_float2(ez, ez);
-            const QAxes w = qaxes(inv, qa, qb);
-            const unsigned live = qpair_live(o, inv, base, w, sx, sy, sz, 0) |
-                                  (qpair_live(o, inv, base, w, sx, sy, sz, 1) << 2);
-            const unsigned leafmask = live & (eb >> 24) & 15u;
-            if (leafmask != 0u) {
-                const unsigned e = ((unsigned)node << 4) | leafmask;
+            // the lowest set bit's index, from a table of two bits per mask
+            const QNode *np = s.qnodes + (gbase + ((0x12131210u >> (2u * gmask)) & 3u));
+            gmask &= gmask - 1u;
+            float4 base, wxy, wz, links;
+            ldg256(&np->base, base, wxy);
+            ldg256(&np->qz, wz, links);
+            const unsigned masks = __float_as_uint(base.w);
+            const unsigned live = qlive(o, inv, base, as_uint4(wxy), as_uint4(wz));
+            const unsigned leaves = live & masks;  // live has slot bits 0-3 only
+            if (leaves != 0u) {
+                const unsigned e = (__float_as_uint(links.y) << 4) | leaves;
                 if (park0 == 0u) park0 = e;
                 else park1 = e;
             }
-            const unsigned im = live & (eb >> 28);
+            const unsigned im = live & (masks >> 4);
             if (im != 0u) {
-                // the first inner child is walked next, the others pushed
-                // (last slot first, so they pop in slot order)
-                const unsigned rest = im & (im - 1u);
-                if (rest & 8u) my_stack[sp++] = ch.w;
-                if (rest & 4u) my_stack[sp++] = ch.z;
-                if (rest & 2u) my_stack[sp++] = ch.y;
-                node = (im & 1u) ? ch.x : (im & 2u) ? ch.y : (im & 4u) ? ch.z : ch.w;
-            } else if (sp > 0) {
-                node = my_stack[--sp];
-            } else {
-                walked = true;
-                if (park0 == 0u) {
+                if (gmask != 0u) {
+                    my_stack[sp * stride] = (int)((gbase << 4) | gmask);
+                    ++sp;
+                }
+                gbase = __float_as_uint(links.x);
+                gmask = im;
+            } else if (gmask == 0u) {
+                if (sp > 0) {
+                    --sp;
+                    const unsigned e = (unsigned)my_stack[sp * stride];
+                    gbase = e >> 4;
+                    gmask = e & 15u;
+                } else if (park0 == 0u) {
                     emit(owner, false);
-                    cur = -1;
+                    busy = false;
                 }
             }
         }
@@ -855,7 +836,7 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
 template <typename Fetch, typename Endpoint, typename Emit>
 __device__ __forceinline__ void trace_pool_f(const DevScene &s, Fetch fetch, int n, int *next, int *stack, int depth,
                                              TraceStats &ts, Endpoint endpoint, Emit emit) {
-    if (s.qnodes != nullptr) trace_quant_loop(s, fetch, n, next, ts, endpoint, emit);
+    if (s.qnodes != nullptr) trace_quant_loop(s, fetch, n, next, stack, ts, endpoint, emit);
     else if (s.wide != nullptr) trace_wide_loop(s, fetch, n, next, ts, endpoint, emit);
     else trace_binary_loop(s, fetch, n, next, stack, depth, ts, endpoint, emit);
 }
