@@ -460,8 +460,9 @@ int32_t host_pack_wide(const rg_aabb_tree_node *src, int32_t n, std::vector<floa
 // bound, e the smallest exponent with D(255) >= its upper bound, and per child
 // the lower code is the largest q with D(q) <= the child's lower bound, the
 // upper code the smallest with D(q) >= its upper bound, so the decoded box
-// contains the child's box.  The host evaluates D with fmaf, which rounds like
-// the device's FMA.  Leaf slots link (as ~index) to leaf records that hold the
+// contains the child's box; every code also bounds its box as the device's
+// walk places planes (host_walk_nodes), with 1/16 code to spare, for which c
+// may lie a step lower and e one higher.  Leaf slots link (as ~index) to leaf records that hold the
 // triangle's exact box from the reference's tree and the triangle itself
 // (host_pack_tris form).
 //
@@ -488,12 +489,22 @@ inline float pow2f(int eb) {
 // D(q) for biased exponent eb and base c
 inline float qdecode(int q, int eb, float c) { return fmaf(8388608.0f + (float)q, pow2f(eb), c); }
 
+// The neighbouring floats of a finite x.
+inline float next_down(float x) {
+    uint32_t u;
+    memcpy(&u, &x, 4);
+    u = (u & 0x7fffffffu) == 0u ? 0x80000001u : (u >> 31) ? u + 1u : u - 1u;
+    memcpy(&x, &u, 4);
+    return x;
+}
+inline float next_up(float x) { return -next_down(-x); }
+
 // The walk's base of an axis: plane q lies at c + (2^15 + q) s in real
 // arithmetic, with c rounded down from the base above.
 inline float walk_base(int eb, float base) {
     const double v = (double)base + (8388608.0 - 32768.0) * (double)pow2f(eb);
     float c = (float)v;
-    while ((double)c > v) c = std::nextafter(c, -INFINITY);
+    while ((double)c > v) c = next_down(c);
     return c;
 }
 inline double walk_plane(int q, int eb, float c) { return (double)c + (32768.0 + q) * (double)pow2f(eb); }
@@ -519,12 +530,13 @@ bool quant_axis(float lo, float hi, float &c, int &eb) {
     eb = std::max(eb, std::min(246, lo_exp - 1 - 23 - 8 + 127));
     for (; eb <= 246; ++eb) {
         const float s = pow2f(eb);
-        float cc = (float)((double)lo - std::ldexp(1.0, eb - 127 + 23));
-        while (fmaf(8388608.0f, s, cc) > lo) cc = std::nextafter(cc, -INFINITY);
-        while (fmaf(8388608.0f, s, std::nextafter(cc, INFINITY)) <= lo) cc = std::nextafter(cc, INFINITY);
-        if (!std::isfinite(cc) || !std::isfinite(qdecode(255, eb, cc))) continue;
+        float cc = (float)((double)lo - 8388608.0 * (double)s);
+        if (!std::isfinite(cc)) continue;
+        while (fmaf(8388608.0f, s, cc) > lo) cc = next_down(cc);
+        while (fmaf(8388608.0f, s, next_up(cc)) <= lo) cc = next_up(cc);
+        if (!std::isfinite(qdecode(255, eb, cc))) continue;
         // a step lower where the walk's plane of code 0 needs it
-        for (int k = 0; k < 2 && !code_below(0, eb, cc, walk_base(eb, cc), lo); ++k) cc = std::nextafter(cc, -INFINITY);
+        for (int k = 0; k < 2 && !code_below(0, eb, cc, walk_base(eb, cc), lo); ++k) cc = next_down(cc);
         const float w = walk_base(eb, cc);
         if (code_below(0, eb, cc, w, lo) && code_above(255, eb, cc, w, hi)) {
             c = cc;
@@ -562,12 +574,14 @@ struct QuantBuilder {
         w[3] = (uint32_t)eb[0] | ((uint32_t)eb[1] << 8) | ((uint32_t)eb[2] << 16) | ((leafbits | innerbits << 4) << 24);
         w[10] = (uint32_t)eb[0] << 23;  // s of x and y as floats (the walk reads them directly)
         w[11] = (uint32_t)eb[1] << 23;
+        float wbase[3];
+        for (int a = 0; a < 3; ++a) wbase[a] = walk_base(eb[a], base[a]);
         for (int k = 0; k < 4 && ok; ++k) {
             const WEntry &c = e[k < n ? k : n - 1];  // an empty slot repeats the last child (ignored)
             for (int a = 0; a < 3; ++a) {
                 // start from the real-valued estimate, then step to the exact codes
-                const double s = std::ldexp(1.0, eb[a] - 127), o = (double)base[a] + 8388608.0 * s;
-                const float wb = walk_base(eb[a], base[a]);
+                const double s = (double)pow2f(eb[a]), o = (double)base[a] + 8388608.0 * s;
+                const float wb = wbase[a];
                 int ql = (int)std::max(0.0, std::min(255.0, std::floor(((double)c.lo[a] - o) / s)));
                 int qh = (int)std::max(0.0, std::min(255.0, std::ceil(((double)c.hi[a] - o) / s)));
                 while (ql > 0 && !code_below(ql, eb[a], base[a], wb, c.lo[a])) --ql;

@@ -1134,7 +1134,7 @@ __global__ void k_count_run(uint32_t *runs) { *runs += 1u; }
 
 size_t ris_smem_bytes(int ppt, int depth, int samples = 1) {
     return (size_t)128 * ppt * samples * (sizeof(rgpool::Ray) + sizeof(float4) + 1) +
-           128 * (size_t)(RG_QSTACK_SHARED ? 16 : RG_STACK_LOCAL ? 0 : depth) * sizeof(int);
+           128 * (size_t)(RG_STACK_LOCAL ? 0 : depth) * sizeof(int);
 }
 
 // Calls f.template operator()<R, MIS>() for the scene's reservoir format.
@@ -1233,7 +1233,7 @@ cudaError_t launch_spatial_unbiased(const DevScene &s, const GBufView &g, const 
         constexpr bool MIS = decltype(tag)::MIS;
         constexpr int BT = RG_UNBIASED_BT;  // block threads: the pixels sharing one ray pool
         const dim3 block(32, BT / 32);
-        const size_t smem = unbiased_smem_bytes(num_neighbors, RG_QSTACK_SHARED ? 16 : RG_STACK_LOCAL ? 0 : s.depth, R, MIS, BT);
+        const size_t smem = unbiased_smem_bytes(num_neighbors, RG_STACK_LOCAL ? 0 : s.depth, R, MIS, BT);
         cudaError_t e = cudaFuncSetAttribute(k_spatial_unbiased<32, R, MIS, BT>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -1267,7 +1267,7 @@ cudaError_t launch_shade(const DevScene &s, const GBufView &g, const rg_reservoi
 cudaError_t launch_visibility_batch(const DevScene &s, const float4 *p1, const float4 *p2, uint8_t *out, int n,
                                     cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    const size_t smem = kVisChunk * (sizeof(rgpool::Ray) + sizeof(float4)) + 128 * (size_t)(RG_QSTACK_SHARED ? 16 : RG_STACK_LOCAL ? 0 : s.depth) * sizeof(int);
+    const size_t smem = kVisChunk * (sizeof(rgpool::Ray) + sizeof(float4)) + 128 * (size_t)(RG_STACK_LOCAL ? 0 : s.depth) * sizeof(int);
     cudaError_t e = cudaFuncSetAttribute(k_visibility_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     k_visibility_batch<<<(unsigned)((n + kVisChunk - 1) / kVisChunk), 128, smem, st>>>(s, p1, p2, out, n);
@@ -1365,7 +1365,7 @@ cudaError_t with_views_kernel(int kind, int variant, bool unbiased, int num_neig
     if (kind == 1) {
         if (!unbiased) return f(k_spatial_biased_views, (size_t)0);
         if (num_neighbors < 0 || num_neighbors > kMaxNeighbors) return cudaErrorInvalidValue;
-        const size_t smem = unbiased_smem_bytes(num_neighbors, RG_QSTACK_SHARED ? 16 : RG_STACK_LOCAL ? 0 : depth);
+        const size_t smem = unbiased_smem_bytes(num_neighbors, RG_STACK_LOCAL ? 0 : depth);
         switch (variant) {
             case 8: return f(k_spatial_unbiased_views<8>, smem);
             case 16: return f(k_spatial_unbiased_views<16>, smem);

@@ -564,9 +564,11 @@ __device__ __forceinline__ uint4 as_uint4(float4 v) {
 // take this walk have |o| <= 2^40 and |d| in [2^-60, 2^60] (ray_fits); A or a
 // product that underflows is far below K.
 // Each axis' near and far code words are picked by the ray's direction sign.
-// Against decoding each plane, subtracting o and multiplying by inv (three
-// packed operations a plane instead of one), 1080p frames with 1.05M
-// triangles: see DESIGN's table for the measured passes.
+// One FMA a plane in place of decoding, subtracting o and multiplying by inv
+// (three packed operations) alone changed little (a 1080p frame with 1.05M
+// triangles 14.53 -> 14.42 ms): the walk was bound by the L1's data pipe; with
+// 256-bit loads and the one-word stack below 12.98 ms (2M segments against the
+// same tree: 1.35 -> 1.31 -> 1.03 ms).
 __device__ __forceinline__ float fma_sat(float a, float b, float c) {
     float y;
     asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
@@ -638,18 +640,17 @@ __device__ __forceinline__ bool qleaf_hit(const QLeaf *lp, f3 o, f3 d, f3 inv) {
 #ifndef RG_QWALK_STEPS
 #define RG_QWALK_STEPS 16
 #endif
-// RG_QSTACK_SHARED: the quantized walk's stack in shared memory.
-#ifndef RG_QSTACK_SHARED
-#define RG_QSTACK_SHARED 0
-#endif
-
 #ifndef RG_UNBIASED_BT
 #define RG_UNBIASED_BT 128
 #endif
 constexpr int kLeafQueueWarps = (RG_UNBIASED_BT > 128 ? RG_UNBIASED_BT : 128) / 32;  // the largest pool block
 
 // Entries of the quantized walk's stack: at most one per level of the copy,
-// and the upload takes copies of up to RG_MAX_TREE_DEPTH / 3 levels.
+// and the upload takes copies of up to RG_MAX_TREE_DEPTH / 3 levels.  In local
+// memory: in shared memory its accesses cost the L1's data pipe less (a batch
+// of 2M segments 0.98 against 1.03 ms), but the unbiased pass, whose blocks
+// hold 15 KB of shared memory already, loses more L1 (a 1080p frame 13.83
+// against 12.98 ms).
 constexpr int kQStack = RG_MAX_TREE_DEPTH / 3;
 
 // The loop over the quantized 4-wide copy (DevScene::qnodes): a node visit
@@ -671,20 +672,13 @@ constexpr int kQStack = RG_MAX_TREE_DEPTH / 3;
 // holding lane has parked (1 KB of shared memory per warp) and tests them with
 // all lanes of the warp.
 template <typename Fetch, typename Endpoint, typename Emit>
-__device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *next, int *stack, TraceStats &ts,
-                                 Endpoint endpoint, Emit emit) {
+__device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *next, TraceStats &ts, Endpoint endpoint,
+                                 Emit emit) {
     constexpr unsigned kFull = 0xffffffffu;
     __shared__ uint32_t s_leafq[kLeafQueueWarps][32 * 8];  // per warp: up to 8 parked leaves per lane
     const int tid = threadIdx.x + threadIdx.y * blockDim.x;
     const int lane = tid & 31;
-#if RG_QSTACK_SHARED
-    int *my_stack = stack + tid;
-    const int stride = blockDim.x * blockDim.y;
-#else
     int my_stack[kQStack];
-    constexpr int stride = 1;
-    (void)stack;
-#endif
     bool busy = false;     // this lane has a segment
     bool retired = false;  // the pool has no segment left for this lane
     int owner = 0, sp = 0, visits = 0;
@@ -811,7 +805,7 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
             const unsigned im = live & (masks >> 4);
             if (im != 0u) {
                 if (gmask != 0u) {
-                    my_stack[sp * stride] = (int)((gbase << 4) | gmask);
+                    my_stack[sp] = (int)((gbase << 4) | gmask);
                     ++sp;
                 }
                 gbase = __float_as_uint(links.x);
@@ -819,7 +813,7 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
             } else if (gmask == 0u) {
                 if (sp > 0) {
                     --sp;
-                    const unsigned e = (unsigned)my_stack[sp * stride];
+                    const unsigned e = (unsigned)my_stack[sp];
                     gbase = e >> 4;
                     gmask = e & 15u;
                 } else if (park0 == 0u) {
@@ -836,7 +830,7 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
 template <typename Fetch, typename Endpoint, typename Emit>
 __device__ __forceinline__ void trace_pool_f(const DevScene &s, Fetch fetch, int n, int *next, int *stack, int depth,
                                              TraceStats &ts, Endpoint endpoint, Emit emit) {
-    if (s.qnodes != nullptr) trace_quant_loop(s, fetch, n, next, stack, ts, endpoint, emit);
+    if (s.qnodes != nullptr) trace_quant_loop(s, fetch, n, next, ts, endpoint, emit);
     else if (s.wide != nullptr) trace_wide_loop(s, fetch, n, next, ts, endpoint, emit);
     else trace_binary_loop(s, fetch, n, next, stack, depth, ts, endpoint, emit);
 }
