@@ -979,21 +979,22 @@ __global__ void __launch_bounds__(128, RG_SHADE_MIN_BLOCKS) k_shade(const ShadeP
 }
 
 // ---------------------------------------------------------------- visibility batch (testVisibility)
-// 128 threads take a chunk of 512 segments into the pool and trace it.
+// A block of T threads takes `chunk` segments into its pool and traces it.
 constexpr int kVisChunk = 512;
 
-__global__ void __launch_bounds__(128, 8) k_visibility_batch(const DevScene s, const float4 *p1, const float4 *p2,
-                                                          uint8_t *out, int n) {
+template <int T>
+__global__ void __launch_bounds__(T, 1024 / T) k_visibility_batch(const DevScene s, const float4 *p1, const float4 *p2,
+                                                                  uint8_t *out, int n, int chunk) {
     extern __shared__ __align__(16) unsigned char smem[];
     rgpool::Ray *pool = reinterpret_cast<rgpool::Ray *>(smem);
-    float4 *endp = reinterpret_cast<float4 *>(pool + kVisChunk);
-    int *stack = reinterpret_cast<int *>(endp + kVisChunk);
+    float4 *endp = reinterpret_cast<float4 *>(pool + chunk);
+    int *stack = reinterpret_cast<int *>(endp + chunk);
     __shared__ int s_next;
     const int tid = threadIdx.x;
-    const int base = blockIdx.x * kVisChunk;
-    const int count = min(kVisChunk, n - base);
+    const int base = blockIdx.x * chunk;
+    const int count = min(chunk, n - base);
     if (tid == 0) s_next = 0;
-    for (int k = tid; k < count; k += 128) {
+    for (int k = tid; k < count; k += T) {
         const float4 a = __ldg(p1 + base + k), b = __ldg(p2 + base + k);
         rgpool::put_ray(pool, k, mk(a.x, a.y, a.z), k);
         endp[k] = b;
@@ -1267,11 +1268,27 @@ cudaError_t launch_shade(const DevScene &s, const GBufView &g, const rg_reservoi
 cudaError_t launch_visibility_batch(const DevScene &s, const float4 *p1, const float4 *p2, uint8_t *out, int n,
                                     cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    const size_t smem = kVisChunk * (sizeof(rgpool::Ray) + sizeof(float4)) + 128 * (size_t)(RG_STACK_LOCAL ? 0 : s.depth) * sizeof(int);
-    cudaError_t e = cudaFuncSetAttribute(k_visibility_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k_visibility_batch<<<(unsigned)((n + kVisChunk - 1) / kVisChunk), 128, smem, st>>>(s, p1, p2, out, n);
-    return cudaGetLastError();
+    auto launch = [&](auto kernel, int threads, int chunk) {
+        const size_t smem = (size_t)chunk * (sizeof(rgpool::Ray) + sizeof(float4)) +
+                            (size_t)threads * (size_t)(RG_STACK_LOCAL ? 0 : s.depth) * sizeof(int);
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kernel<<<(unsigned)((n + chunk - 1) / chunk), threads, smem, st>>>(s, p1, p2, out, n, chunk);
+        return cudaGetLastError();
+    };
+    // A batch of up to 32 segments a warp for 8 warps an SM goes out as single
+    // warps of 4 to 32 segments, so that it reaches every SM; a larger one as
+    // blocks of 128 to 512 segments.  Blocks of 512 at every size took 48 us
+    // for 512 segments, 50 us for 39,000 (780 triangles; 163 and 194 us with
+    // 1.05M); now 16 and 20 (45 and 86) us.  4, 8 or 16 warps an SM differ by
+    // 2 % up to 20,000 segments; 16 is 15 % slower at 39,000.
+    constexpr int kWarps = 152 * 8;
+    if (n <= kWarps * 32) {
+        const int per_warp = (n + kWarps - 1) / kWarps;
+        return launch(k_visibility_batch<32>, 32, per_warp < 4 ? 4 : per_warp);
+    }
+    const int per_block = (n + 152 * 8 - 1) / (152 * 8);
+    return launch(k_visibility_batch<128>, 128, per_block < 128 ? 128 : per_block < kVisChunk ? per_block : kVisChunk);
 }
 
 // ---------------------------------------------------------------- views: parameter records and launches
