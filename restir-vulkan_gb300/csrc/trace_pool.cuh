@@ -594,11 +594,14 @@ __device__ __forceinline__ unsigned qlive(f3 o, f3 inv, const float4 &base, cons
     const float2 ay2 = make_float2(ay, ay), az2 = make_float2(az, az);
     unsigned live = 0u;
 #pragma unroll
-    for (unsigned k = 0; k < 4; ++k) {
+    for (int j = 3; j >= 0; --j) {
+        const unsigned k = (unsigned)j;
         const float tnx = fma_sat(code_float(nx, k), ax, bnx), tfx = fma_sat(code_float(fx, k), ax, bfx);
         const float2 ty = __ffma2_rn(make_float2(code_float(ny, k), code_float(fy, k)), ay2, by);
         const float2 tz = __ffma2_rn(make_float2(code_float(nz, k), code_float(fz, k)), az2, bz);
-        if (max3f(tnx, ty.x, tz.x) < min3f(tfx, ty.y, tz.y)) live |= 1u << k;
+        // entry < exit as the sign of their difference (no NaN here; equal
+        // values give +0), shifted into the mask: one ALU operation a child
+        live = __funnelshift_l(__float_as_uint(max3f(tnx, ty.x, tz.x) - min3f(tfx, ty.y, tz.y)), live, 1);
     }
     return live;
 }
@@ -634,12 +637,22 @@ __device__ __forceinline__ bool qleaf_hit(const QLeaf *lp, f3 o, f3 d, f3 inv) {
     return hit && rgm::ray_tri(mk(b.z, b.w, c.x), mk(c.y, c.z, c.w), mk(e.x, e.y, e.z), o, d);
 }
 
-// Node visits per walking lane per pass through the quantized walk's warp
-// loop (with two leaf slots lanes stop less often: 8, 12, 16, 24, 32 steps
-// give 5.60, 5.49, 5.44, 5.63, 5.99 ms per 1080p unbiased pass).
+// The quantized walk's schedule (as RG_WALK_STEPS, RG_FETCH_MIN and
+// RG_LEAF_MIN).  1080p frames with 1.05M / 100k triangles: 16, 12, 10, 8, 6
+// steps with minimums 4 and 2 give 12.67 / 11.55, 12.52 / 11.14, 12.55 /
+// 10.95, 12.57 / 10.85, 12.72 / 10.77 ms; 8 steps with a leaf minimum of 1
+// (a phase as soon as a lane cannot walk on) 12.50 / 10.76, and a fetch
+// minimum of 6 with it 12.41 / 10.68.
 #ifndef RG_QWALK_STEPS
-#define RG_QWALK_STEPS 16
+#define RG_QWALK_STEPS 8
 #endif
+#ifndef RG_QFETCH_MIN
+#define RG_QFETCH_MIN 6
+#endif
+#ifndef RG_QLEAF_MIN
+#define RG_QLEAF_MIN 1
+#endif
+
 #ifndef RG_UNBIASED_BT
 #define RG_UNBIASED_BT 128
 #endif
@@ -669,13 +682,13 @@ constexpr int kQStack = RG_MAX_TREE_DEPTH / 3;
 // Each lane may hold two parked leaf sets (record of slot 0 << 4 | slot mask,
 // the record modulo 2^27), so it
 // keeps walking past its first leaves; the leaf phase lists the leaves every
-// holding lane has parked (1 KB of shared memory per warp) and tests them with
+// holding lane has parked (a byte each in shared memory) and tests them with
 // all lanes of the warp.
 template <typename Fetch, typename Endpoint, typename Emit>
 __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *next, TraceStats &ts, Endpoint endpoint,
                                  Emit emit) {
     constexpr unsigned kFull = 0xffffffffu;
-    __shared__ uint32_t s_leafq[kLeafQueueWarps][32 * 8];  // per warp: up to 8 parked leaves per lane
+    __shared__ uint8_t s_leafq[kLeafQueueWarps][32 * 8];  // per warp: up to 8 parked leaves per lane
     const int tid = threadIdx.x + threadIdx.y * blockDim.x;
     const int lane = tid & 31;
     int my_stack[kQStack];
@@ -690,7 +703,7 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
         const bool idle = !retired && !busy;
         const unsigned m_idle = __ballot_sync(kFull, idle);
         const unsigned m_busy = __ballot_sync(kFull, busy);
-        if (m_idle != 0u && (__popc(m_idle) >= RG_FETCH_MIN || m_busy == 0u)) {
+        if (m_idle != 0u && (__popc(m_idle) >= RG_QFETCH_MIN || m_busy == 0u)) {
             if (idle) {
                 ts.visits += (unsigned)visits;  // the finished segment's node visits
                 visits = 0;
@@ -720,12 +733,13 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
         const bool blocked = busy && (gmask == 0u || park1 != 0u);
         const unsigned m_block = __ballot_sync(kFull, blocked);
         const unsigned m_walk = __ballot_sync(kFull, busy && !blocked);
-        if (m_block != 0u && (__popc(m_block) >= RG_LEAF_MIN || m_walk == 0u)) {
-            // the holders' leaves go to the warp's queue ((lane << 27) |
-            // record), and every lane tests queued leaves, a chunk of 32 at a
-            // time, with the owning lane's ray taken by shuffles; a ray's
-            // remaining leaves are skipped once one of its leaves hits
-            uint32_t *q = s_leafq[tid >> 5];
+        if (m_block != 0u && (__popc(m_block) >= RG_QLEAF_MIN || m_walk == 0u)) {
+            // the holders' leaves go to the warp's queue (lane << 3 | set << 2
+            // | slot, a byte each, which leaves the SM more L1), and every
+            // lane tests queued leaves, a chunk of 32 at a time, with the
+            // owning lane's set and ray taken by shuffles; a ray's remaining
+            // leaves are skipped once one of its leaves hits
+            uint8_t *q = s_leafq[tid >> 5];
             const bool holder = busy && park0 != 0u;
             const int cnt = holder ? __popc(park0 & 15u) + __popc(park1 & 15u) : 0;
             int incl = cnt;
@@ -741,7 +755,7 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
                 for (int slot = 0; slot < 2; ++slot) {
                     const unsigned e = slot == 0 ? park0 : park1;
                     for (unsigned m = e & 15u; m != 0u; m &= m - 1u)
-                        q[at++] = ((unsigned)lane << 27) | (((e >> 4) + (unsigned)(__ffs(m) - 1)) & 0x7ffffffu);
+                        q[at++] = (uint8_t)((lane << 3) | (slot << 2) | (__ffs(m) - 1));
                 }
             }
             __syncwarp();
@@ -749,14 +763,16 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
             for (int base = 0; base < total; base += 32) {
                 const int j = base + lane;
                 const unsigned e = j < total ? q[j] : 0u;
-                const int src = (int)(e >> 27);
+                const int src = (int)(e >> 3);
+                const unsigned set0 = __shfl_sync(kFull, park0, src), set1 = __shfl_sync(kFull, park1, src);
+                const unsigned rec = (((e & 4u) ? set1 : set0) >> 4) + (e & 3u);
                 const f3 so = mk(__shfl_sync(kFull, o.x, src), __shfl_sync(kFull, o.y, src), __shfl_sync(kFull, o.z, src));
                 const f3 sd = mk(__shfl_sync(kFull, d.x, src), __shfl_sync(kFull, d.y, src), __shfl_sync(kFull, d.z, src));
                 const f3 si =
                     mk(__shfl_sync(kFull, inv.x, src), __shfl_sync(kFull, inv.y, src), __shfl_sync(kFull, inv.z, src));
                 bool h = false;
                 if (j < total && ((hits >> src) & 1u) == 0u) {
-                    h = qleaf_hit(s.qleaves + (e & 0x7ffffffu), so, sd, si);
+                    h = qleaf_hit(s.qleaves + (rec & 0x7ffffffu), so, sd, si);
                     ++ts.tri_tests;
                 }
                 hits |= __reduce_or_sync(kFull, h ? 1u << src : 0u);
