@@ -219,15 +219,16 @@ __device__ __forceinline__ void add_sample(ResV<R, MIS> &r, float4 pos_lum, floa
     }
 }
 // add_sample with the reservoir-update uniforms drawn beforehand (u[j] is the
-// draw update_at would take for sample j): the same arithmetic.
+// draw update_at would take for sample j) and the sample's W left to
+// finish_samples: the same arithmetic on the same values, with the division
+// of W made once a sample instead of once a candidate.
 template <int R, bool MIS>
-__device__ __forceinline__ void add_sample_u(ResV<R, MIS> &r, float4 pos_lum, float4 nrm, int32_t idx, float p_hat,
-                                             float sample_p, const float (&u)[R]) {
+__device__ __forceinline__ void add_sample_u(ResV<R, MIS> &r, uint32_t (&at)[R], float4 pos_lum, float4 nrm, int32_t idx,
+                                             float p_hat, float sample_p, const float (&u)[R]) {
     const float weight = p_hat / sample_p;
     r.m += 1u;
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-        const float w = (r.sum_w[j] + weight) / ((float)r.m * p_hat);
         r.sum_w[j] += weight;
         const float replace = weight / r.sum_w[j];
         if (u[j] < replace) {
@@ -235,10 +236,17 @@ __device__ __forceinline__ void add_sample_u(ResV<R, MIS> &r, float4 pos_lum, fl
             r.nrm[j] = nrm;
             r.idx[j] = idx;
             r.p_hat[j] = p_hat;
-            r.w[j] = w;
+            r.w[j] = r.sum_w[j];  // the sum with this candidate
+            at[j] = r.m;          // and the count
             if (MIS) r.sum_phat[j] += p_hat;
         }
     }
+}
+template <int R, bool MIS>
+__device__ __forceinline__ void finish_samples(ResV<R, MIS> &r, const uint32_t (&at)[R]) {
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+        if (at[j] != 0u) r.w[j] = r.w[j] / ((float)at[j] * r.p_hat[j]);
 }
 // reservoir.glsl:44-64.  With MIS the reference passes other's sumPHat where
 // updateReservoirAt takes w and other's w where it takes sumPHat (:55-60);
@@ -295,13 +303,17 @@ __device__ __forceinline__ void count_block_rays(const DevScene &s, int rays, co
 #define RG_SMEM_CARVEOUT -1
 #endif
 
-// Pixels per thread of the single-view launch (the batched one is tuned):
-// 3 (32 x 12 tiles) measured fastest at 1080p among 2 to 6 (3.33 ms against
-// 3.34, 3.48, 3.44 and 4.21 ms for 2, 4, 5 and 6).
+// Pixels per thread of the single-view launch (the batched one is tuned): 3
+// (32 x 12 tiles) for large frames, whose blocks then have enough segments to
+// keep their lanes at work to the end (1280x720: 1.36 ms for RIS, two biased
+// passes and shading, against 1.42 and 1.56 with 2 and 1); 1 while one-pixel
+// blocks all fit on the chip at once, where a thread's pixels one after the
+// other are the time (256x256, whole frame: 0.109 ms against 0.195).
 #ifndef RG_RIS_PPT
 #define RG_RIS_PPT 3
 #endif
 constexpr int kRisPpt = RG_RIS_PPT;
+constexpr uint64_t kRisSmallFrame = 152 * 8 * 128;  // pixels: 8 blocks of 128 on every SM
 
 struct InitialParams {
     DevScene s;
@@ -363,6 +375,9 @@ __device__ __forceinline__ ResV<R, MIS> ris(const DevScene &s, const Texel &t, f
         int col = imin((int)((float)count * r1), count - 1);
         float4 cc = __ldg(&s.alias[col].col), own = __ldg(&s.alias[col].own_pos), ali = __ldg(&s.alias[col].alias_pos);
         const float4 nrm0 = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t at[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) at[j] = 0u;
         for (uint32_t c = 0; c < count_c; ++c) {
             float u[R];
 #pragma unroll
@@ -383,13 +398,14 @@ __device__ __forceinline__ ResV<R, MIS> ris(const DevScene &s, const Texel &t, f
             const float prob = keep ? cc.z : cc.w;
             const int32_t lidx = keep ? col : __float_as_int(cc.y);
             const float ph = eval_phat_px(pp, xyz(pos_lum), xyz(nrm0), false, pos_lum.w);
-            add_sample_u(r, pos_lum, nrm0, lidx, ph, prob, u);
+            add_sample_u(r, at, pos_lum, nrm0, lidx, ph, prob, u);
             r2 = r2n;
             col = coln;
             cc = ccn;
             own = ownn;
             ali = alin;
         }
+        finish_samples(r, at);
         if (flags & RG_FLAG_FINAL_RIS_WEIGHT) {
 #pragma unroll
             for (int j = 0; j < R; ++j)
@@ -464,21 +480,28 @@ __device__ __forceinline__ ResV<R, MIS> ris(const DevScene &s, const Texel &t, f
 #ifndef RG_RIS_MIN_BLOCKS
 #define RG_RIS_MIN_BLOCKS 8
 #endif
+// Two samples per reservoir: 80 registers and fewer spills beat two more
+// blocks (641x359 with MIS: 1.27 ms a frame at 8 blocks, 1.21 at 6).
+#ifndef RG_RIS_MIN_BLOCKS2
+#define RG_RIS_MIN_BLOCKS2 6
+#endif
 // The pass over one 32 x (4*PPT) pixel tile (tile coordinates bx, by); with
 // R samples per reservoir each pixel traces R visibility segments.
 template <int PPT, int R, bool MIS>
 __device__ __forceinline__ void initial_temporal_tile(const InitialParams &p, int bx, int by) {
     constexpr int kTile = 128 * PPT;
     extern __shared__ __align__(16) unsigned char smem[];
-    rgpool::Ray *pool = reinterpret_cast<rgpool::Ray *>(smem);
-    float4 *endp = reinterpret_cast<float4 *>(pool + kTile * R);  // sample position per (pixel slot, sample)
-    uint8_t *shadow = reinterpret_cast<uint8_t *>(endp + kTile * R);
+    // The pool holds owner tags only: a segment's start is re-read from the
+    // G-buffer and its end from the pixel's reservoir in `out` when a lane
+    // takes it.
+    uint16_t *pool = reinterpret_cast<uint16_t *>(smem);
+    uint8_t *shadow = reinterpret_cast<uint8_t *>(pool + kTile * R);
     int *stack = reinterpret_cast<int *>(shadow + kTile * R);
     __shared__ int s_count, s_next;
     const int tid = threadIdx.x + threadIdx.y * 32;
     if (tid == 0) { s_count = 0; s_next = 0; }
-    __syncthreads();
     const DevScene &s = p.s;
+    __syncthreads();
     const int W = (int)p.u.screen_size[0], H = (int)p.u.screen_size[1];
     const int x = bx * 32 + threadIdx.x;
     const int y0 = by * (4 * PPT) + threadIdx.y;
@@ -486,51 +509,57 @@ __device__ __forceinline__ void initial_temporal_tile(const InitialParams &p, in
     const bool vis = (p.u.flags & RG_FLAG_VISIBILITY_REUSE) != 0;
     const bool swap_fix = (p.u.flags & RG_FLAG_MIS_SWAP_FIX) != 0;
     uint64_t rng_state[PPT];
-#pragma unroll
+    // not unrolled: three copies of the candidate loop missed the instruction
+    // cache (a 1080p frame 13.10 -> 12.81 ms)
+#pragma unroll 1
     for (int j = 0; j < PPT; ++j) {
         const int y = y0 + 4 * j;
         const bool valid = x < W && y < H;
+        const size_t i = (size_t)y * (size_t)W + (size_t)x;
         bool want = false;
-        f3 wpos = mk(0.f, 0.f, 0.f);
-        float4 lpos[R];
-#pragma unroll
-        for (int q = 0; q < R; ++q) lpos[q] = make_float4(0.f, 0.f, 0.f, 0.f);
         rng_state[j] = 0;
         if (valid) {
-            const size_t i = (size_t)y * (size_t)W + (size_t)x;
             Texel t;
             load_texel(p.cur, i, t);
             const float albedo_lum = luminance(t.albedo.x, t.albedo.y, t.albedo.z);
             Pcg rng = pcg_seed((uint64_t)p.u.frame, (uint64_t)((uint32_t)y * 10007u + (uint32_t)x));
-            const bool zero_normal = !(dot(t.normal, t.normal) != 0.0f);
-            const ResV<R, MIS> r = ris<R, MIS>(s, t, albedo_lum, cam, p.u.initial_light_sample_count, zero_normal,
+            want = dot(t.normal, t.normal) != 0.0f;
+            const ResV<R, MIS> r = ris<R, MIS>(s, t, albedo_lum, cam, p.u.initial_light_sample_count, !want,
                                                p.u.flags, p.learned, i, rng);
             store_resv(p.out, i, r);
             rng_state[j] = rng.state;
-            // visibility reuse :147-160; a background pixel's (zero normal) sample is the
-            // zero sample, for which zeroing w and sumWeights changes nothing: no ray
-            want = vis && !zero_normal;
-            wpos = t.wpos;
-#pragma unroll
-            for (int q = 0; q < R; ++q) lpos[q] = make_float4(r.pos_lum[q].x, r.pos_lum[q].y, r.pos_lum[q].z, 0.0f);
         }
+        // visibility reuse :147-160; a background pixel's (zero normal) sample is the
+        // zero sample, for which zeroing w and sumWeights changes nothing: no ray
+        const bool ray = vis && want;
 #pragma unroll
         for (int q = 0; q < R; ++q) {
             const int owner = (j * 128 + tid) * R + q;
-            shadow[owner] = want ? 0 : 2;  // 2: no segment
-            endp[owner] = lpos[q];
-            const int slot = rgpool::append_slot(&s_count, want);
-            if (want) rgpool::put_ray(pool, slot, wpos, owner);
+            shadow[owner] = ray ? 0 : 2;  // 2: no segment
+            const int slot = rgpool::append_slot(&s_count, ray);
+            if (ray) pool[slot] = (uint16_t)owner;
         }
     }
     __syncthreads();
+    auto pixel_of = [&](int owner) {  // pool owner -> pixel
+        const int e = owner / R, tt = e & 127;
+        return (size_t)(by * (4 * PPT) + (tt >> 5) + 4 * (e >> 7)) * (size_t)W + (size_t)(bx * 32 + (tt & 31));
+    };
+    using L = ResLayout<R, MIS>;
+    const float4 *own = reinterpret_cast<const float4 *>(p.out);  // coherent loads: this block wrote it
     rgpool::TraceStats ts;
-    rgpool::trace_pool(
-        s, pool, s_count, &s_next, stack, s.depth, ts,
-        [&](int owner) { const float4 e = endp[owner]; return mk(e.x, e.y, e.z); },
+    rgpool::trace_pool_f(
+        s,
+        [&](int slot, f3 &p1) {
+            const int owner = pool[slot];
+            p1 = load_wpos(p.cur, pixel_of(owner));
+            return owner;
+        },
+        s_count, &s_next, stack, s.depth, ts,
+        [&](int owner) { return xyz(own[pixel_of(owner) * L::kWords + (owner % R) * L::kSample4]); },
         [&](int owner, bool hit) { shadow[owner] = hit ? 1 : 0; });
     __syncthreads();
-#pragma unroll
+#pragma unroll 1
     for (int j = 0; j < PPT; ++j) {
         const int y = y0 + 4 * j;
         if (x >= W || y >= H) continue;
@@ -545,8 +574,7 @@ __device__ __forceinline__ void initial_temporal_tile(const InitialParams &p, in
                 if (MIS) r.sum_phat[q] = 0.0f;
             }
             if (p.vc.out) {
-                const float4 e = endp[owner];
-                vcache_put(p.vc, (size_t)q * p.vc.n + i, load_wpos(p.cur, i), mk(e.x, e.y, e.z),
+                vcache_put(p.vc, (size_t)q * p.vc.n + i, load_wpos(p.cur, i), xyz(r.pos_lum[q]),
                            shadow[owner] == 2 ? -1 : (int)shadow[owner]);
             }
         }
@@ -595,7 +623,7 @@ __device__ __forceinline__ void initial_temporal_tile(const InitialParams &p, in
 }
 
 template <int PPT, int R, bool MIS>
-__global__ void __launch_bounds__(128, RG_RIS_MIN_BLOCKS) k_initial_temporal(const InitialParams p) {
+__global__ void __launch_bounds__(128, R == 1 ? RG_RIS_MIN_BLOCKS : RG_RIS_MIN_BLOCKS2) k_initial_temporal(const InitialParams p) {
     initial_temporal_tile<PPT, R, MIS>(p, blockIdx.x, blockIdx.y);
 }
 
@@ -677,7 +705,7 @@ __host__ __device__ inline size_t unbiased_smem_bytes(int K, int depth, int R = 
     size_t b = (size_t)bt * (size_t)R * sizeof(float4);
     b += (size_t)bt * kp * sizeof(uint32_t);
     b += (size_t)bt * kp * (mis ? (size_t)R : 1) * sizeof(uint32_t);
-    b += (size_t)bt * slots * (size_t)R * sizeof(int);
+    b += (size_t)bt * slots * (size_t)R * sizeof(uint16_t);
     b += ((size_t)bt * slots * (size_t)R + 15) & ~(size_t)15;
     b += (size_t)bt * (size_t)depth * sizeof(int);
     return b;
@@ -700,7 +728,7 @@ __device__ __forceinline__ void spatial_unbiased_tile(const SpatialParams &p, in
     uint32_t *nidx = reinterpret_cast<uint32_t *>(endp + BT * R);                  // [K][BT]
     uint32_t *nm = nidx + BT * kp;                                                 // [K][BT]
     float *nsp = reinterpret_cast<float *>(nm);                                     // MIS: [R][K][BT]
-    int *pool = reinterpret_cast<int *>(nm + BT * kp * (MIS ? R : 1));             // owners, [R][K+1][BT] slots
+    uint16_t *pool = reinterpret_cast<uint16_t *>(nm + BT * kp * (MIS ? R : 1));   // owners, [R][K+1][BT] slots
     uint8_t *flag = reinterpret_cast<uint8_t *>(pool + BT * slots * R);            // [R][K+1][BT]
     int *stack = reinterpret_cast<int *>(flag + ((BT * slots * R + 15) & ~15));
     __shared__ int s_count, s_next;
@@ -806,7 +834,7 @@ __device__ __forceinline__ void spatial_unbiased_tile(const SpatialParams &p, in
         flag[(q * slots + K) * BT + tid] = own_known == 1 ? 1 : 0;
         const bool own = valid && vis && own_known < 0;
         const int slot = rgpool::append_range(&s_count, own ? 1 : 0);
-        if (own) pool[slot] = (q * slots + K) * BT + tid;
+        if (own) pool[slot] = (uint16_t)((q * slots + K) * BT + tid);
     }
     __syncthreads();
 #pragma unroll
@@ -814,7 +842,7 @@ __device__ __forceinline__ void spatial_unbiased_tile(const SpatialParams &p, in
         int slot = rgpool::append_range(&s_count, __popc(wantm[q]));
         for (uint32_t m = wantm[q]; m != 0u; m &= m - 1u) {
             const int k = __ffs(m) - 1;
-            pool[slot++] = (q * slots + k) * BT + tid;
+            pool[slot++] = (uint16_t)((q * slots + k) * BT + tid);
         }
     }
     __syncthreads();
@@ -1134,8 +1162,8 @@ __global__ void k_advance_frames(InitialParams *ip, SpatialParams *sp, int n_vie
 __global__ void k_count_run(uint32_t *runs) { *runs += 1u; }
 
 size_t ris_smem_bytes(int ppt, int depth, int samples = 1) {
-    return (size_t)128 * ppt * samples * (sizeof(rgpool::Ray) + sizeof(float4) + 1) +
-           128 * (size_t)(RG_STACK_LOCAL ? 0 : depth) * sizeof(int);
+    const size_t tags = ((size_t)128 * ppt * samples * (sizeof(uint16_t) + 1) + 3) & ~(size_t)3;
+    return tags + 128 * (size_t)(RG_STACK_LOCAL ? 0 : depth) * sizeof(int);
 }
 
 // Calls f.template operator()<R, MIS>() for the scene's reservoir format.
@@ -1184,15 +1212,18 @@ cudaError_t launch_initial_temporal(const DevScene &s, const GBufView &cur, cons
     return with_format(s, [&](auto tag) {
         constexpr int R = decltype(tag)::R;
         constexpr bool MIS = decltype(tag)::MIS;
-        constexpr int ppt = R == 1 ? kRisPpt : 2;  // pool size per block kept near the single-sample one
-        const dim3 block(32, 4);
-        const dim3 grid((u.screen_size[0] + 31u) / 32u, (u.screen_size[1] + 4u * ppt - 1u) / (4u * ppt));
-        const size_t smem = ris_smem_bytes(ppt, s.depth, R);
-        cudaError_t e = cudaFuncSetAttribute(k_initial_temporal<ppt, R, MIS>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        k_initial_temporal<ppt, R, MIS><<<grid, block, smem, st>>>(p);
-        return cudaGetLastError();
+        constexpr int many = R == 1 ? kRisPpt : 2;  // pool size per block kept near the single-sample one
+        auto launch = [&](auto kernel, unsigned ppt) {
+            const dim3 grid((u.screen_size[0] + 31u) / 32u, (u.screen_size[1] + 4u * ppt - 1u) / (4u * ppt));
+            const size_t smem = ris_smem_bytes((int)ppt, s.depth, R);
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+            kernel<<<grid, dim3(32, 4), smem, st>>>(p);
+            return cudaGetLastError();
+        };
+        const uint64_t px = (uint64_t)u.screen_size[0] * u.screen_size[1];
+        if (px <= kRisSmallFrame) return launch(k_initial_temporal<1, R, MIS>, 1u);
+        return launch(k_initial_temporal<many, R, MIS>, (unsigned)many);
     });
 }
 

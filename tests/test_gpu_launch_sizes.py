@@ -1,5 +1,5 @@
-"""Batches of shadow segments at the sizes where their launch shape changes,
-and the G-buffer of cameras whose rays leave the packed slab test.
+"""Batches of shadow segments and RIS frames at the sizes where their launch
+shape changes, and the G-buffer of cameras whose rays leave the packed slab test.
 
 Bar: bit-exact.  A segment's answer does not depend on its batch (the large
 batch is pinned against the oracle in test_gpu_visibility.py); G-buffer planes
@@ -51,3 +51,34 @@ def test_gbuffer_of_axis_aligned_cameras(ctx, cuda, scene, size, target):
     dev = g.to_host()
     for k, v in host.items():
         assert np.array_equal(v.view(np.uint8), dev[k].view(np.uint8)), k
+
+
+@pytest.mark.parametrize("samples,mis", [(1, 0), (1, 1), (2, 0), (2, 1)])
+@pytest.mark.parametrize("rows", [1, 100, 310, 311])
+def test_ris_frames_on_both_sides_of_the_shape_rule(ctx, cuda, scene, samples, mis, rows):
+    """A pixel's RIS result depends on its coordinates and texel only, so the
+    top rows of a frame just above the rule's pixel count (several pixels per
+    thread) equal those of a frame with only these rows (one per thread)."""
+    from restir_gb300.passes import DeviceGBuffer, reservoirs
+    w, h = 501, 313
+    assert w * 310 < 152 * 8 * 128 < w * 311
+    s = scene.view(scene.cameras[0], w, h)
+    ctx.upload_scene(s)
+    ctx.set_reservoir_format(samples, mis)
+    try:
+        nbytes = ctx.reservoir_bytes()
+        g = DeviceGBuffer(w, h)
+        ctx.trace_gbuffer(s.cameras[0], g)
+        u = s.uniforms(0)
+        full = reservoirs(w * h, nbytes=nbytes)
+        ctx.initial_temporal(g, None, None, full, u)
+        top = DeviceGBuffer(w, rows)
+        for k, t in top.planes.items():
+            t.copy_(g.planes[k][:rows])
+        u.screen_size[:] = [w, rows]
+        part = reservoirs(w * rows, nbytes=nbytes)
+        ctx.initial_temporal(top, None, None, part, u)
+        assert cuda.equal(part, full[:w * rows])
+        assert int((full != 0).sum()) > 0
+    finally:
+        ctx.set_reservoir_format(1, 0)
