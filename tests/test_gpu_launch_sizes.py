@@ -82,3 +82,33 @@ def test_ris_frames_on_both_sides_of_the_shape_rule(ctx, cuda, scene, samples, m
         assert int((full != 0).sum()) > 0
     finally:
         ctx.set_reservoir_format(1, 0)
+
+
+def test_reservoir_buffers_at_16_byte_alignment(ctx, cuda, scene):
+    """The spatial and shading passes read reservoirs by 256-bit loads where
+    the buffer is 32-byte aligned; a caller's need only be 16-byte aligned."""
+    from restir_gb300.passes import DeviceGBuffer, reservoirs
+    w, h = 77, 45
+    s = scene.view(scene.cameras[0], w, h)
+    ctx.upload_scene(s)
+    g = DeviceGBuffer(w, h)
+    ctx.trace_gbuffer(s.cameras[0], g)
+    u = s.uniforms(0)
+    n = w * h
+    r0 = reservoirs(n)
+    ctx.initial_temporal(g, None, None, r0, u)
+    raw = cuda.zeros(n * 16 + 4, dtype=cuda.int32, device="cuda")
+    shifted = raw[4:].view(n, 16)
+    shifted.copy_(r0)
+    assert r0.data_ptr() % 32 == 0 and shifted.data_ptr() % 32 == 16
+    outs = []
+    for src in (r0, shifted):
+        ctx.initial_temporal(g, None, None, reservoirs(n), u)
+        a, b = reservoirs(n), reservoirs(n)
+        ctx.spatial_unbiased(g, src, a, u, 5, 0)
+        ctx.spatial_biased(g, src, b, u, 0)
+        img = cuda.zeros((h, w, 4), dtype=cuda.float32, device="cuda")
+        ctx.shade(g, src, s.lighting_uniforms(0), img)
+        outs.append((a, b, img.view(cuda.int32)))
+    for p, q in zip(*outs):
+        assert cuda.equal(p, q)
