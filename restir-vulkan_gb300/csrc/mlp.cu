@@ -6,10 +6,9 @@
 // cluster logit layer in chunks of 64 clusters, double-buffered in tensor
 // memory so that the MMA of chunk c+1 runs under the epilogue of chunk c.
 // Weight tiles arrive by cp.async from bf16 images that are already in the MMA
-// operand layout.  Logits never leave the SM.  Three epilogues:
+// operand layout.  Logits never leave the SM.  Exponentials are 2^x on the MUFU
+// unit with the log2(e) scale folded into one FMA per logit.  Two epilogues:
 //   kLse     log-sum-exp, arg-max and its probability per row;
-// Exponentials are 2^x on the MUFU unit with the log2(e) scale folded into
-// one FMA per logit.
 //   kSample  the learned-branch candidates: each row walks its softmax CDF
 //            once with its uniforms drawn as ascending order statistics; a
 //            uniform's column inside the 32-column piece that holds it is
@@ -17,11 +16,13 @@
 //            probability is the width of its interval.  (The uniform-branch
 //            candidates, a light and q of its cluster, are written at the
 //            end of kLse.)
-//   kGrad    for training: dz = d(loss)/d(logits) = (softmax - onehot) / n
-//            per chunk into a bf16 tile, then dh3 += dz W4^T on the tensor
-//            cores (accumulated in tensor memory over the chunks), and the
-//            cross-entropy loss.  dz never leaves the SM; dW4 and db4 come
-//            from k_mlp_dw4, which recomputes the logits chunk by chunk.
+// Training runs kLse with the hidden activations saved, then from h3:
+//   k_mlp_grad  dz = d(loss)/d(logits) = (softmax - onehot) / n per chunk into
+//            a bf16 tile, then dh3 += dz W4^T on the tensor cores, and the
+//            cross-entropy loss;
+//   k_mlp_dw4   dW4 and db4, from the logits recomputed chunk by chunk (dz
+//            never leaves the SM);
+//   k_mlp_backward_rows  the hidden layers.
 // Every wait on the tensor core is bounded; a CTA whose wait runs out records
 // an error, waits (bounded) for its last MMA, frees its tensor memory and
 // leaves.  At most four CTAs share an SM: each holds 128 tensor-memory
@@ -43,7 +44,6 @@ constexpr int kRows = 128;                 // rows (pixels) per CTA
 constexpr int kChunkN = mlp::kChunkN;      // clusters per logit MMA chunk
 constexpr uint32_t kMaxPolls = 1u << 26;   // bounded mbarrier waits
 constexpr int kTmemCols = 2 * kChunkN;    // two chunk accumulators; the hidden layers use them first
-constexpr int kTmemColsGrad = 4 * kChunkN;  // kGrad: plus the dh3 accumulator (64 columns), rounded up
 
 // shared-memory map (bytes)
 constexpr int kOffX = 0;                               // x tile, 128 x 16 bf16
@@ -55,16 +55,11 @@ constexpr int kOffB = kOffW3 + mlp::kH * mlp::kH * 2;  // two chunk tiles, 128 x
 constexpr int kChunkBytes = kChunkN * mlp::kH * 2;
 constexpr int kOffBias = kOffB + 2 * kChunkBytes;      // b1 | b2 | b3
 constexpr int kSmemUsed = kOffBias + 3 * mlp::kH * 4;
-// kGrad: the logit-gradient tile (128 rows x 64 clusters, K-major over
-// clusters) and two W4 chunk tiles (64 hidden x 64 clusters) for dh3 += dz W4^T
-constexpr int kOffDz = (kSmemUsed + 1023) / 1024 * 1024;
-constexpr int kOffWk = kOffDz + kRows * kChunkN * 2;
 constexpr int kWkBytes = mlp::kH * kChunkN * 2;
-constexpr int kSmemGrad = kOffWk + 2 * kWkBytes;
 constexpr int kSmemMin = 52 * 1024;                    // caps residency at four CTAs per SM (TMEM: 4 x 128 columns)
 constexpr int kWeightImgBytes = (mlp::kH * mlp::kIn + 2 * mlp::kH * mlp::kH) * 2;
 
-enum { kLse = 0, kSample = 1, kGrad = 2 };
+enum { kLse = 0, kSample = 1 };
 
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
@@ -166,13 +161,9 @@ struct FusedParams {
     const int32_t *rows;       // pixel of each row; nullptr: row = pixel
     int n;
     float4 *stat;              // per row: lse, arg-max cluster (int bits), its probability, 0
-    // training (kLse with save != 0, kGrad)
+    // training (kLse with save != 0)
     int save;
     __nv_bfloat16 *x, *h1, *h2, *h3;  // [n x 16], [n x 64] x 3
-    const int32_t *target;     // cluster per row, -1: no target
-    float *dh3;                // [n x 64] FP32: d(loss)/d(h3)
-    float inv_n;
-    float *loss_sum;
     // sampling
     mlp::Candidate *cand;      // [n x kCand]
     uint32_t frame;
@@ -220,6 +211,50 @@ __device__ __forceinline__ void store8(__nv_bfloat16 *dst, const float *v) {
     *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(b);
 }
 
+// One 32-column piece of a row's logit gradient, (softmax - onehot) / n as
+// bf16 into the K-major dz tile: v holds the logits, nl2 = -lse * log2(e),
+// hit = target - first column or kNoTarget (the row's gradient is 0).  Only the piece that holds a row's target pays for the one-hot:
+// testing every column took 445 instructions a piece instead of about 150.
+// Returns the target's logit where the piece holds it, else 0.
+constexpr int kNoTarget = INT32_MIN;
+__device__ __forceinline__ float grad_piece(unsigned char *dztile, int row, int col0, const float2 (&v)[16], float nl2,
+                                            float inv_n, int hit) {
+    float2 d[16];
+    const float2 l2 = make_float2(kLog2e, kLog2e), o2 = make_float2(nl2, nl2), s2 = make_float2(inv_n, inv_n);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const float2 t = __ffma2_rn(v[k], l2, o2);
+        d[k] = __fmul2_rn(make_float2(ex2(t.x), ex2(t.y)), s2);
+    }
+    float zt = 0.0f;
+    if ((unsigned)hit < 32u) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            if (i == hit) {
+                zt = col(v, i);
+                const float g = (ex2(__fmaf_rn(zt, kLog2e, nl2)) - 1.0f) * inv_n;
+                if (i & 1) d[i >> 1].y = g;
+                else d[i >> 1].x = g;
+            }
+    }
+    if (hit == kNoTarget) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) d[k] = make_float2(0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int q = 0; q < 32; q += 8) {
+        uint4 w;
+        uint32_t *b = reinterpret_cast<uint32_t *>(&w);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const __nv_bfloat162 h = __float22bfloat162_rn(d[q / 2 + k]);
+            b[k] = *reinterpret_cast<const uint32_t *>(&h);
+        }
+        *reinterpret_cast<uint4 *>(dztile + umma::kmajor_offset(row, col0 + q, kChunkN)) = w;
+    }
+    return zt;
+}
+
 // Bounded wait for an MMA commit; warp-uniform result.
 __device__ __forceinline__ bool mma_wait(uint64_t *mbar, uint32_t parity) {
     bool w = umma::mbar_wait(mbar, parity, kMaxPolls);
@@ -230,9 +265,9 @@ __device__ __forceinline__ bool mma_wait(uint64_t *mbar, uint32_t parity) {
 template <int kMode, bool kViews>
 __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ uint64_t mbar_layer, mbar_chunk[2], mbar_dh;
+    __shared__ uint64_t mbar_layer, mbar_chunk[2];
     __shared__ uint32_t tmem_base;
-    constexpr int kCols = kMode == kGrad ? kTmemColsGrad : kTmemCols;
+    constexpr int kCols = kTmemCols;
     const int tid = threadIdx.x, warp = tid >> 5;
     const int row = blockIdx.x * kRows + tid;
     const bool valid = row < p.n;
@@ -270,19 +305,11 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
     float *bias = reinterpret_cast<float *>(smem + kOffBias);
     const unsigned char *w4img = reinterpret_cast<const unsigned char *>(p.pd.w4t);
 
-    unsigned char *dztile = smem + kOffDz;
-    unsigned char *wkslot[2] = {smem + kOffWk, smem + kOffWk + kWkBytes};
-    const unsigned char *w4kimg = reinterpret_cast<const unsigned char *>(p.pd.w4k);
-
     // weights and the first two logit chunks start moving
     copy_bytes(smem + kOffW1, reinterpret_cast<const unsigned char *>(p.pd.w123img), kWeightImgBytes);
     copy_bytes(btile[0], w4img, kChunkBytes);
-    if (kMode == kGrad) copy_bytes(wkslot[0], w4kimg, kWkBytes);
     cp_async_commit();
-    if (nch > 1) {
-        copy_bytes(btile[1], w4img + kChunkBytes, kChunkBytes);
-        if (kMode == kGrad) copy_bytes(wkslot[1], w4kimg + kWkBytes, kWkBytes);
-    }
+    if (nch > 1) copy_bytes(btile[1], w4img + kChunkBytes, kChunkBytes);
     cp_async_commit();
     for (int i = tid; i < 3 * mlp::kH; i += blockDim.x) {
         const size_t b = i < mlp::kH ? L.b1 : i < 2 * mlp::kH ? L.b2 : L.b3;
@@ -293,7 +320,6 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
         umma::mbar_init(&mbar_layer, 1);
         umma::mbar_init(&mbar_chunk[0], 1);
         umma::mbar_init(&mbar_chunk[1], 1);
-        umma::mbar_init(&mbar_dh, 1);
     }
     {
         float x[mlp::kIn];
@@ -378,25 +404,19 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
     // ---- logit chunks
     float m = -INFINITY, s = 0.0f;  // kLse: running max and sum
     int amax = 0;
-    float lse = 0.0f, cum = 0.0f;   // kSample / kGrad
+    float lse = 0.0f, cum = 0.0f;   // kSample
     float next_u = INFINITY;  // no uniform left (cum never exceeds it, even when it overflows)
     int amax_row = 0;
     float qmax_row = 0.0f;
-    int target = -1;
-    float zt = 0.0f;
-    if (kMode != kLse && valid) {
+    if (kMode == kSample && valid) {
         const float4 st = p.stat[row];
         lse = st.x;
         amax_row = __float_as_int(st.y);
         qmax_row = st.z;
-        if (kMode == kSample) {
-            if (n_u > 0) {
-                u_prev = next_order_stat(rng, 0.0f, n_u);
-                k_u = 1;
-                next_u = u_prev;
-            }
-        } else {
-            target = p.target[row];
+        if (n_u > 0) {
+            u_prev = next_order_stat(rng, 0.0f, n_u);
+            k_u = 1;
+            next_u = u_prev;
         }
     }
     const float nl2 = -lse * kLog2e;
@@ -487,7 +507,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
                 } else {
                     s = __fmaf_rn(sp, ex2((mp - m) * kLog2e), s);
                 }
-            } else if (kMode == kSample) {
+            } else {
                 exp_piece(v, nl2);
                 const float end = cum + sum32(v);
                 // the uniforms below `end` belong to this piece
@@ -524,41 +544,10 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
                     } while (next_u < end);
                 }
                 cum = end;
-            } else {  // kGrad: the gradient rows go to the dz tile (bf16)
-                float d[32];
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const float z = col(v, i);
-                    const float pr = ex2(__fmaf_rn(z, kLog2e, nl2));
-                    const bool hit = (col0 + i) == target;
-                    if (hit) zt = z;
-                    d[i] = target < 0 ? 0.0f : (pr - (hit ? 1.0f : 0.0f)) * p.inv_n;
-                }
-#pragma unroll
-                for (int q = 0; q < 32; q += 8) put8(dztile, tid, piece * 32 + q, kChunkN, d + q);
             }
         }
         }  // w
         umma::fence_before_sync();
-        if (kMode == kGrad) {
-            // dh3 += dz_tile . W4[:, chunk]^T once every row's gradient is in the tile
-            umma::fence_proxy_async();
-            ok = __syncthreads_and(ok && ok_warp) != 0;
-            umma::fence_after_sync();
-            if (!ok) break;
-            if (tid == 0) {
-                umma::mma_chunk(tmem + (uint32_t)(2 * kChunkN), dztile, wkslot[c & 1], kChunkN, kRows, mlp::kH, c > 0);
-                umma::mma_commit(&mbar_dh);
-                last_mbar = &mbar_dh;
-                last_parity = (uint32_t)(c & 1);
-            }
-            const bool w2 = mma_wait(&mbar_dh, (uint32_t)(c & 1));
-            ok_warp = ok_warp && w2;
-            if (w2 && c + 2 < nch) {  // the slot is free once this product completed
-                copy_bytes(wkslot[c & 1], w4kimg + (size_t)(c + 2) * kWkBytes, kWkBytes);
-                cp_async_commit();
-            }
-        }
     }
     ok = __syncthreads_and(ok && ok_warp) != 0;
     if (!ok) {
@@ -617,35 +606,182 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
                     p.cand[(size_t)row * mlp::kCand + j] = mlp::Candidate{l, ex2(__fmaf_rn(z, kLog2e, nl))};
                 }
             }
-        } else if (kMode == kSample) {
+        } else {
             // uniforms beyond the rounded CDF total: the most probable cluster
             while (next_u < INFINITY) take(amax_row, qmax_row);
         }
-    }
-    if (kMode == kGrad && ok) {
-        float d[64];
-        umma::tmem_ld32(tmem + (uint32_t)(2 * kChunkN), warp, 0, *reinterpret_cast<float(*)[32]>(d));
-        umma::tmem_ld32(tmem + (uint32_t)(2 * kChunkN), warp, 32, *reinterpret_cast<float(*)[32]>(d + 32));
-        if (valid) {
-            float4 *dst = reinterpret_cast<float4 *>(p.dh3 + (size_t)row * mlp::kH);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) dst[j] = make_float4(d[4 * j], d[4 * j + 1], d[4 * j + 2], d[4 * j + 3]);
-        }
-    }
-    if (kMode == kGrad && ok) {
-        float l = (valid && target >= 0) ? lse - zt : 0.0f;
-        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-        if ((tid & 31) == 0 && l != 0.0f) atomicAdd(p.loss_sum, l);
     }
     umma::fence_before_sync();
     __syncthreads();
     if (warp == 0) umma::tmem_dealloc(tmem, kCols);
 }
 
+// ---------------------------------------------------------------- training: dh3 and the loss
+// One CTA per 128 rows: the forward pass from the saved h3, then per chunk of
+// 64 clusters z = h3 . W4[:, chunk] on the tensor cores, dz = (softmax -
+// onehot) / n as bf16 into a tile, and dh3 += dz W4[:, chunk]^T, accumulated
+// in tensor memory.  Bound by the latency of that chain, so four CTAs share an
+// SM (128 tensor-memory columns and 49 KB each): the weight tiles are single,
+// each refilled under the epilogue that follows its product, and a chunk has
+// one barrier, after which both products are issued (its dh3 and the next z).
+// 65,536 rows and 4096 clusters are 512 CTAs: with two an SM (88 KB, two
+// barriers a chunk, the hidden layers run again, the one-hot tested at every
+// column) they took 0.315 ms in two rounds; now 0.154 ms in one.
+constexpr int kGOffH = 0;                                  // h3 tile, 128 x 64 bf16
+constexpr int kGOffDz = kGOffH + kRows * mlp::kH * 2;      // dz tile, 128 x 64 (K-major over clusters)
+constexpr int kGOffB = kGOffDz + kRows * kChunkN * 2;      // W4^T chunk (cluster x hidden)
+constexpr int kGOffWk = kGOffB + kChunkBytes;              // W4 chunk (hidden x cluster)
+constexpr int kGradSmem = kGOffWk + kWkBytes;
+constexpr int kGradTmem = 2 * kChunkN;                     // z, dh3
+
+struct GradParams {
+    mlp::ProposalDev pd;
+    const __nv_bfloat16 *h3;   // [n x 64]
+    const float4 *stat;        // per row: lse first
+    const int32_t *target;     // cluster per row, -1: no target
+    int n;
+    float inv_n;
+    float *dh3;                // [n x 64] FP32: d(loss)/d(h3)
+    float *loss_sum;
+    int *err;
+};
+
+__global__ void __launch_bounds__(128, 4) k_mlp_grad(const GradParams p) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ uint64_t mbar_z, mbar_dh;
+    __shared__ uint32_t tmem_base;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int row = blockIdx.x * kRows + tid;
+    const bool valid = row < p.n;
+    const int nch = p.pd.c / kChunkN;
+    unsigned char *htile = smem + kGOffH, *dztile = smem + kGOffDz, *btile = smem + kGOffB, *wk = smem + kGOffWk;
+    const unsigned char *w4img = reinterpret_cast<const unsigned char *>(p.pd.w4t);
+    const unsigned char *w4kimg = reinterpret_cast<const unsigned char *>(p.pd.w4k);
+    copy_bytes(btile, w4img, kChunkBytes);
+    copy_bytes(wk, w4kimg, kWkBytes);
+    // the saved h3 rows, eight threads a row
+    for (int e = tid; e < kRows * 8; e += kRows) {
+        const int r = e >> 3, j = e & 7;
+        unsigned char *dst = htile + umma::kmajor_offset(r, 8 * j, mlp::kH);
+        if (blockIdx.x * kRows + r < p.n)
+            cp_async16(dst, reinterpret_cast<const unsigned char *>(p.h3) +
+                                ((size_t)(blockIdx.x * kRows + r) * mlp::kH + 8 * j) * 2);
+        else
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
+    }
+    cp_async_commit();
+    if (warp == 0) umma::tmem_alloc(&tmem_base, kGradTmem);
+    if (tid == 0) {
+        umma::mbar_init(&mbar_z, 1);
+        umma::mbar_init(&mbar_dh, 1);
+    }
+    float lse = 0.0f, zt = 0.0f;
+    int target = -1;
+    if (valid) {
+        lse = p.stat[row].x;
+        target = p.target[row];
+    }
+    const float nl2 = -lse * kLog2e;
+    cp_async_wait_all();
+    umma::fence_proxy_async();
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tmem = tmem_base;
+    bool ok = true, ok_warp = true;
+    uint64_t *last_mbar = nullptr;  // thread 0's most recent commit
+    uint32_t last_parity = 0;
+    if (tid == 0) {
+        umma::mma_chunk(tmem, htile, btile, mlp::kH, kRows, kChunkN, false);
+        umma::mma_commit(&mbar_z);
+        last_mbar = &mbar_z;
+    }
+    for (int c = 0; c < nch; ++c) {
+        const bool w = mma_wait(&mbar_z, (uint32_t)(c & 1));
+        ok_warp = ok_warp && w;
+        if (w) {
+            if (c + 1 < nch) {  // the product has read its weights
+                copy_bytes(btile, w4img + (size_t)(c + 1) * kChunkBytes, kChunkBytes);
+                cp_async_commit();
+            }
+            const float4 *be = reinterpret_cast<const float4 *>(p.pd.b4e + c * kChunkN);
+            uint32_t raw[2][32];
+            umma::tmem_ld32_issue(tmem, warp, 0, raw[0]);
+#pragma unroll
+            for (int piece = 0; piece < kChunkN / 32; ++piece) {
+                umma::tmem_ld32_wait(raw[piece & 1]);
+                if (piece + 1 < kChunkN / 32) umma::tmem_ld32_issue(tmem, warp, (piece + 1) * 32, raw[(piece + 1) & 1]);
+                const uint32_t(&rw)[32] = raw[piece & 1];
+                float2 v[16];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const float4 b = __ldg(be + piece * 8 + q);
+                    v[2 * q] = __fadd2_rn(make_float2(__uint_as_float(rw[4 * q]), __uint_as_float(rw[4 * q + 1])),
+                                          make_float2(b.x, b.y));
+                    v[2 * q + 1] = __fadd2_rn(
+                        make_float2(__uint_as_float(rw[4 * q + 2]), __uint_as_float(rw[4 * q + 3])), make_float2(b.z, b.w));
+                }
+                if (piece == 0 && c > 0) {  // the previous chunk's product has read the dz tile and its weights
+                    const bool w2 = mma_wait(&mbar_dh, (uint32_t)((c - 1) & 1));
+                    ok_warp = ok_warp && w2;
+                    if (w2) {
+                        copy_bytes(wk, w4kimg + (size_t)c * kWkBytes, kWkBytes);
+                        cp_async_commit();
+                    }
+                }
+                zt += grad_piece(dztile, tid, piece * 32, v, nl2, p.inv_n,
+                                 target < 0 ? kNoTarget : target - (c * kChunkN + piece * 32));
+            }
+        }
+        cp_async_wait_all();
+        umma::fence_proxy_async();
+        umma::fence_before_sync();
+        ok = __syncthreads_and(ok_warp) != 0;
+        umma::fence_after_sync();
+        if (!ok) break;
+        if (tid == 0) {
+            umma::mma_chunk(tmem + (uint32_t)kChunkN, dztile, wk, kChunkN, kRows, mlp::kH, c > 0);
+            umma::mma_commit(&mbar_dh);
+            last_mbar = &mbar_dh;
+            last_parity = (uint32_t)(c & 1);
+            if (c + 1 < nch) {
+                umma::mma_chunk(tmem, htile, btile, mlp::kH, kRows, kChunkN, false);
+                umma::mma_commit(&mbar_z);
+                last_mbar = &mbar_z;
+                last_parity = (uint32_t)((c + 1) & 1);
+            }
+        }
+    }
+    if (ok) ok_warp = mma_wait(&mbar_dh, (uint32_t)((nch - 1) & 1)) && ok_warp;
+    ok = __syncthreads_and(ok && ok_warp) != 0;
+    if (!ok) {
+        if (tid == 0) {
+            atomicAdd(p.err, 1);
+            if (last_mbar) umma::mbar_wait(last_mbar, last_parity, kMaxPolls);
+        }
+        cp_async_wait_all();
+    } else {
+        float d[64];
+        umma::tmem_ld32(tmem + (uint32_t)kChunkN, warp, 0, *reinterpret_cast<float(*)[32]>(d));
+        umma::tmem_ld32(tmem + (uint32_t)kChunkN, warp, 32, *reinterpret_cast<float(*)[32]>(d + 32));
+        if (valid) {
+            float4 *dst = reinterpret_cast<float4 *>(p.dh3 + (size_t)row * mlp::kH);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) dst[j] = make_float4(d[4 * j], d[4 * j + 1], d[4 * j + 2], d[4 * j + 3]);
+        }
+        float l = (valid && target >= 0) ? lse - zt : 0.0f;
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if ((tid & 31) == 0 && l != 0.0f) atomicAdd(p.loss_sum, l);
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) umma::tmem_dealloc(tmem, kGradTmem);
+}
+
 // ---------------------------------------------------------------- dW4, db4
 // One CTA per (chunk of 64 clusters, slice of row tiles).  Per 128-row tile:
 // the chunk's logits z = h3 . W4[:, chunk] on the tensor cores, the bf16
-// gradient dz = (softmax - onehot) / n as in kGrad (same formula, so the same
+// gradient dz = (softmax - onehot) / n as in k_mlp_grad (same formula, so the same
 // values), then dW[0..63] += h3^T dz and dW[64] += 1^T dz (db4) as one MMA
 // with M = 128 and K = the tile's 128 rows, accumulated in tensor memory; the
 // CTA adds its 65 x 64 result to the gradient with atomics at the end.
@@ -658,9 +794,6 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
 // bytes either way, with SBO the step between core matrices along M/N and
 // LBO the step along K.  The tiles sit at the start of a 64 KB allocation, so
 // every address those descriptors can form stays inside it.
-#ifndef RG_DW4_SLICE_CTAS
-#define RG_DW4_SLICE_CTAS 4
-#endif
 struct Dw4Params {
     mlp::ProposalDev pd;
     const __nv_bfloat16 *h3;   // [n x 64]
@@ -720,22 +853,33 @@ __global__ void __launch_bounds__(128, 3) k_mlp_dw4(const Dw4Params p) {
     uint32_t last_parity = 0;
     const float4 *be = reinterpret_cast<const float4 *>(p.pd.b4e + chunk * kChunkN);
     const uint32_t ht_a = umma::smem_addr(ht), dz_a = umma::smem_addr(dzt), bz_a = umma::smem_addr(bz);
+    // the next tile's rows travel in registers under this tile's work
+    uint4 hrow[8];  // 16 bytes of rows tid / 8 + 16 j, eight threads a row
+    auto fetch_row = [&](int t) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int row = t * kRows + (tid >> 3) + 16 * j;
+            hrow[j] = t < t1 && row < p.n
+                          ? __ldg(reinterpret_cast<const uint4 *>(p.h3 + (size_t)row * mlp::kH + 8 * (tid & 7)))
+                          : make_uint4(0, 0, 0, 0);
+        }
+    };
+    if (ok) fetch_row(t0);
     for (int t = t0; t < t1 && ok; ++t) {
         const int k = t - t0;
-        if (k > 0) ok_warp = ok_warp && mma_wait(&mbar_w, (uint32_t)((k - 1) & 1));  // previous tile's operands free
         const int row = t * kRows + tid;
         const bool valid = row < p.n;
+        float lse = 0.0f;
+        int target = -1;
         if (valid) {
-            const unsigned char *src = reinterpret_cast<const unsigned char *>(p.h3 + (size_t)row * mlp::kH);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) cp_async16(ht + umma::kmajor_offset(tid, 8 * j, kDwHCols), src + 16 * j);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                *reinterpret_cast<uint4 *>(ht + umma::kmajor_offset(tid, 8 * j, kDwHCols)) = make_uint4(0, 0, 0, 0);
+            target = p.target[row];
+            lse = p.stat[row].x;
         }
-        cp_async_commit();
-        cp_async_wait_all();
+        const float nl2 = -lse * kLog2e;
+        if (k > 0) ok_warp = ok_warp && mma_wait(&mbar_w, (uint32_t)((k - 1) & 1));  // previous tile's operands free
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4 *>(ht + umma::kmajor_offset((tid >> 3) + 16 * j, 8 * (tid & 7), kDwHCols)) = hrow[j];
         umma::fence_proxy_async();
         umma::fence_before_sync();
         ok = __syncthreads_and(ok_warp) != 0;
@@ -751,34 +895,26 @@ __global__ void __launch_bounds__(128, 3) k_mlp_dw4(const Dw4Params p) {
             last_mbar = &mbar_z;
             last_parity = (uint32_t)(k & 1);
         }
+        fetch_row(t + 1);
         const bool w = mma_wait(&mbar_z, (uint32_t)(k & 1));
         ok_warp = ok_warp && w;
         if (w) {
-            float lse = 0.0f;
-            int target = -1;
-            if (valid) {
-                lse = p.stat[row].x;
-                target = p.target[row];
-            }
-            const float nl2 = -lse * kLog2e;
 #pragma unroll
             for (int piece = 0; piece < kChunkN / 32; ++piece) {
-                float v[32];
-                umma::tmem_ld32(tmem, warp, piece * 32, v);
+                uint32_t raw[32];
+                umma::tmem_ld32_issue(tmem, warp, piece * 32, raw);
+                umma::tmem_ld32_wait(raw);
+                float2 v[16];
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     const float4 b = __ldg(be + piece * 8 + q);
-                    v[4 * q] += b.x; v[4 * q + 1] += b.y; v[4 * q + 2] += b.z; v[4 * q + 3] += b.w;
+                    v[2 * q] = __fadd2_rn(make_float2(__uint_as_float(raw[4 * q]), __uint_as_float(raw[4 * q + 1])),
+                                          make_float2(b.x, b.y));
+                    v[2 * q + 1] = __fadd2_rn(
+                        make_float2(__uint_as_float(raw[4 * q + 2]), __uint_as_float(raw[4 * q + 3])), make_float2(b.z, b.w));
                 }
-                float d[32];
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const int col = chunk * kChunkN + piece * 32 + i;
-                    const float pr = ex2(__fmaf_rn(v[i], kLog2e, nl2));
-                    d[i] = target < 0 ? 0.0f : (pr - (col == target ? 1.0f : 0.0f)) * p.inv_n;
-                }
-#pragma unroll
-                for (int q = 0; q < 32; q += 8) put8(dzt, tid, piece * 32 + q, kChunkN, d + q);
+                grad_piece(dzt, tid, piece * 32, v, nl2, p.inv_n,
+                           target < 0 ? kNoTarget : target - (chunk * kChunkN + piece * 32));
             }
         }
         umma::fence_proxy_async();
@@ -839,160 +975,143 @@ struct BackParams {
 };
 
 constexpr int kTileStride = 68;  // floats per row of the row tiles (16-byte rows, conflict-free)
+constexpr int kBackThreads = 256;
 // W2^T, W3^T, the da tile and the layer-input tile (128 rows each)
 constexpr int kBackSmem = (2 * mlp::kH * mlp::kH + 2 * 128 * kTileStride) * 4;
 
-// One row per thread: dh_{l-1} = W_l da_l for 16 outputs at a time, the
-// weights W_l^T in shared memory (row k: W_l[0..63][k]) read as broadcast
-// float4s, the products as packed FP32x2 FMAs.
-__device__ __forceinline__ void back_matvec(const float *wt, const float (&da)[mlp::kH], int i0, float (&o)[16]) {
-    float2 acc[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = make_float2(0.0f, 0.0f);
-#pragma unroll
-    for (int k = 0; k < mlp::kH; ++k) {
-        const float2 d = make_float2(da[k], da[k]);
-        const float4 *w = reinterpret_cast<const float4 *>(wt + k * mlp::kH + i0);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float4 w4 = w[j];
-            acc[2 * j] = __ffma2_rn(make_float2(w4.x, w4.y), d, acc[2 * j]);
-            acc[2 * j + 1] = __ffma2_rn(make_float2(w4.z, w4.w), d, acc[2 * j + 1]);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        o[2 * j] = acc[j].x;
-        o[2 * j + 1] = acc[j].y;
-    }
+// Two columns of FP32 FMAs: acc[j] += a * b[j].
+__device__ __forceinline__ void fma4(float2 (&acc)[2], float a, const float4 &b) {
+    const float2 a2 = make_float2(a, a);
+    acc[0] = __ffma2_rn(a2, make_float2(b.x, b.y), acc[0]);
+    acc[1] = __ffma2_rn(a2, make_float2(b.z, b.w), acc[1]);
 }
 
+// The rows of a bf16 matrix with W columns into the tile's first W columns.
 template <int W>
-__device__ __forceinline__ void load_bf16_row(const __nv_bfloat16 *src, float (&v)[W]) {
-    const uint4 *s4 = reinterpret_cast<const uint4 *>(src);
-#pragma unroll
-    for (int j = 0; j < W / 8; ++j) {
-        const uint4 w = s4[j];
+__device__ __forceinline__ void load_tile(float *tile, const __nv_bfloat16 *src, int row0, int n) {
+    for (int e = threadIdx.x; e < 128 * (W / 8); e += kBackThreads) {
+        const int r = e / (W / 8), c = (e % (W / 8)) * 8;
+        uint4 w = make_uint4(0, 0, 0, 0);
+        if (row0 + r < n) w = *reinterpret_cast<const uint4 *>(src + (size_t)(row0 + r) * W + c);
         const __nv_bfloat162 *b = reinterpret_cast<const __nv_bfloat162 *>(&w);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 f = __bfloat1622float2(b[i]);
-            v[8 * j + 2 * i] = f.x;
-            v[8 * j + 2 * i + 1] = f.y;
-        }
+        float4 *d = reinterpret_cast<float4 *>(tile + r * kTileStride + c);
+        const float2 f0 = __bfloat1622float2(b[0]), f1 = __bfloat1622float2(b[1]), f2 = __bfloat1622float2(b[2]),
+                     f3 = __bfloat1622float2(b[3]);
+        d[0] = make_float4(f0.x, f0.y, f1.x, f1.y);
+        d[1] = make_float4(f2.x, f2.y, f3.x, f3.y);
     }
 }
 
-// gW[i][k0 .. k0 + 2*NP) += sum over the tile's rows of in[r][i] * da[r][k]
-template <int NP>
-__device__ __forceinline__ void tile_outer(const float *in_t, const float *da_t, int i, int k0, float *gw) {
-    float2 acc[NP];
-#pragma unroll
-    for (int j = 0; j < NP; ++j) acc[j] = make_float2(0.0f, 0.0f);
-#pragma unroll 4
-    for (int r = 0; r < 128; ++r) {
-        const float a = in_t[r * kTileStride + i];
-        const float2 a2 = make_float2(a, a);
-        const float4 *d = reinterpret_cast<const float4 *>(da_t + r * kTileStride + k0);
-#pragma unroll
-        for (int j = 0; j < NP / 2; ++j) {
-            const float4 d4 = d[j];
-            acc[2 * j] = __ffma2_rn(a2, make_float2(d4.x, d4.y), acc[2 * j]);
-            acc[2 * j + 1] = __ffma2_rn(a2, make_float2(d4.z, d4.w), acc[2 * j + 1]);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < NP; ++j) {
-        atomicAdd(gw + i * mlp::kH + k0 + 2 * j, acc[j].x);
-        atomicAdd(gw + i * mlp::kH + k0 + 2 * j + 1, acc[j].y);
-    }
-}
-
-// The hidden layers' backward pass for 128 rows per block, one row per
-// thread: da3 = dh3 relu'(h3); for l = 3, 2, 1: db_l += column sums of da_l,
-// dW_l += in_l^T da_l (in_3 = h2, in_2 = h1, in_1 = x; from tiles of the
-// block's rows in shared memory), and da_{l-1} = (W_l da_l) relu'(h_{l-1}),
+// The hidden layers' backward pass for 128 rows per block: da3 = dh3
+// relu'(h3); for l = 3, 2, 1: db_l += column sums of da_l, dW_l += in_l^T da_l
+// (in_3 = h2, in_2 = h1, in_1 = x), and da_{l-1} = (W_l da_l) relu'(h_{l-1}),
 // FP32 with the bf16 weights of the forward pass.  The weight and bias
 // gradients are added to the output with atomics, once per block.
-__global__ void __launch_bounds__(128, 2) k_mlp_backward_rows(const BackParams p) {
+//
+// Bound by shared-memory reads, so a thread owns a register tile of each
+// product: 4 x 4 of dW (two 16-byte reads for 16 FMAs a row) and 8 rows x 4
+// columns of da (12 reads for 128 FMAs every four terms).  One row per thread
+// read nine and four values for 32 and 16 FMAs: 65,536 rows took 0.241 ms, now
+// 0.107.
+__global__ void __launch_bounds__(kBackThreads, 2) k_mlp_backward_rows(const BackParams p) {
     extern __shared__ __align__(16) float bsm[];
     float *wt2 = bsm, *wt3 = bsm + mlp::kH * mlp::kH;
     float *dt = bsm + 2 * mlp::kH * mlp::kH, *it = dt + 128 * kTileStride;  // da tile, layer-input tile
-    for (int e = threadIdx.x; e < 2 * mlp::kH * mlp::kH; e += blockDim.x) {
+    const int t = threadIdx.x, row0 = blockIdx.x * 128;
+    for (int e = t; e < 2 * mlp::kH * mlp::kH; e += kBackThreads) {
         const int layer = e / (mlp::kH * mlp::kH), f = e % (mlp::kH * mlp::kH);
         const int i = f / mlp::kH, k = f % mlp::kH;  // W[i][k]
         (layer ? wt3 : wt2)[k * mlp::kH + i] = __bfloat162float(p.w123[mlp::kIn * mlp::kH + e]);
     }
-    const int t = threadIdx.x;
-    const int r = blockIdx.x * blockDim.x + t;
-    const bool valid = r < p.n;
-    const size_t ro = (size_t)(valid ? r : 0) * mlp::kH;
-    float da[mlp::kH];
-    if (valid) {
-        float h[mlp::kH];
-        load_bf16_row(p.h3 + ro, h);
-        const float4 *g = reinterpret_cast<const float4 *>(p.dh3 + ro);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const float4 v = g[j];
-            da[4 * j] = h[4 * j] > 0.0f ? v.x : 0.0f;
-            da[4 * j + 1] = h[4 * j + 1] > 0.0f ? v.y : 0.0f;
-            da[4 * j + 2] = h[4 * j + 2] > 0.0f ? v.z : 0.0f;
-            da[4 * j + 3] = h[4 * j + 3] > 0.0f ? v.w : 0.0f;
+    load_tile<mlp::kH>(it, p.h3, row0, p.n);
+    __syncthreads();
+    for (int e = t; e < 128 * 16; e += kBackThreads) {  // da3
+        const int r = e >> 4, c = (e & 15) * 4;
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row0 + r < p.n) {
+            g = *reinterpret_cast<const float4 *>(p.dh3 + (size_t)(row0 + r) * mlp::kH + c);
+            const float4 h = *reinterpret_cast<const float4 *>(it + r * kTileStride + c);
+            g = make_float4(h.x > 0.0f ? g.x : 0.0f, h.y > 0.0f ? g.y : 0.0f, h.z > 0.0f ? g.z : 0.0f,
+                            h.w > 0.0f ? g.w : 0.0f);
         }
-    } else {
-#pragma unroll
-        for (int j = 0; j < mlp::kH; ++j) da[j] = 0.0f;
+        *reinterpret_cast<float4 *>(dt + r * kTileStride + c) = g;
     }
+    const int c0 = (t & 15) * 4, g0 = t >> 4;  // this thread's 4 columns, its group of 16 threads
 #pragma unroll 1
     for (int layer = 3; layer >= 1; --layer) {
-        float hin[mlp::kH];  // this layer's input row (x uses the first 16)
-        if (layer > 1) {
-            if (valid) load_bf16_row(layer == 3 ? p.h2 + ro : p.h1 + ro, hin);
-            else
-#pragma unroll
-                for (int j = 0; j < mlp::kH; ++j) hin[j] = 0.0f;
-        } else {
-            float x[mlp::kIn];
-            if (valid) load_bf16_row(p.x + (size_t)r * mlp::kIn, x);
-            else
-#pragma unroll
-                for (int j = 0; j < mlp::kIn; ++j) x[j] = 0.0f;
-#pragma unroll
-            for (int j = 0; j < mlp::kH; ++j) hin[j] = j < mlp::kIn ? x[j] : 0.0f;
-        }
-        __syncthreads();  // the previous layer's tiles are no longer read (first pass: the weights are in)
-        float4 *drow = reinterpret_cast<float4 *>(dt + t * kTileStride);
-        float4 *irow = reinterpret_cast<float4 *>(it + t * kTileStride);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            drow[j] = make_float4(da[4 * j], da[4 * j + 1], da[4 * j + 2], da[4 * j + 3]);
-            irow[j] = make_float4(hin[4 * j], hin[4 * j + 1], hin[4 * j + 2], hin[4 * j + 3]);
-        }
+        __syncthreads();  // da is complete and the input tile no longer read
+        if (layer == 3) load_tile<mlp::kH>(it, p.h2, row0, p.n);
+        else if (layer == 2) load_tile<mlp::kH>(it, p.h1, row0, p.n);
+        else load_tile<mlp::kIn>(it, p.x, row0, p.n);
         __syncthreads();
-        {  // db_l: thread t sums half the rows of column t % 64
-            const int col = t & 63, half = t >> 6;
+        if (t < 128) {  // db_l: thread t sums half the rows of column t % 64
+            const int c = t & 63, half = t >> 6;
             float sum = 0.0f;
 #pragma unroll 8
-            for (int q = 0; q < 64; ++q) sum += dt[(half * 64 + q) * kTileStride + col];
-            atomicAdd((layer == 3 ? p.gb3 : layer == 2 ? p.gb2 : p.gb1) + col, sum);
+            for (int q = 0; q < 64; ++q) sum += dt[(half * 64 + q) * kTileStride + c];
+            atomicAdd((layer == 3 ? p.gb3 : layer == 2 ? p.gb2 : p.gb1) + c, sum);
         }
-        if (layer > 1) {
-            tile_outer<16>(it, dt, t >> 1, (t & 1) * 32, layer == 3 ? p.gw3 : p.gw2);
-            float nx[mlp::kH];
-            const float *wt = layer == 3 ? wt3 : wt2;
-            const float *own = it + t * kTileStride;  // this row's input: the ReLU mask
+        if (layer == 1) {  // dW1, 16 x 64: one row of four columns a thread
+            float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll 4
+            for (int r = 0; r < 128; ++r)
+                fma4(acc, it[r * kTileStride + g0], *reinterpret_cast<const float4 *>(dt + r * kTileStride + c0));
+            float *dst = p.gw1 + g0 * mlp::kH + c0;
+            atomicAdd(dst, acc[0].x);
+            atomicAdd(dst + 1, acc[0].y);
+            atomicAdd(dst + 2, acc[1].x);
+            atomicAdd(dst + 3, acc[1].y);
+            break;
+        }
+        {  // dW_l, 64 x 64: rows 4 g0 .. 4 g0 + 3, columns c0 .. c0 + 3
+            float2 acc[4][2];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                float o[16];
-                back_matvec(wt, da, 16 * c, o);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) nx[16 * c + j] = own[16 * c + j] > 0.0f ? o[j] : 0.0f;
+            for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = make_float2(0.f, 0.f);
+#pragma unroll 4
+            for (int r = 0; r < 128; ++r) {
+                const float4 a = *reinterpret_cast<const float4 *>(it + r * kTileStride + 4 * g0);
+                const float4 d = *reinterpret_cast<const float4 *>(dt + r * kTileStride + c0);
+                fma4(acc[0], a.x, d);
+                fma4(acc[1], a.y, d);
+                fma4(acc[2], a.z, d);
+                fma4(acc[3], a.w, d);
             }
+            float *gw = (layer == 3 ? p.gw3 : p.gw2) + 4 * g0 * mlp::kH + c0;
 #pragma unroll
-            for (int j = 0; j < mlp::kH; ++j) da[j] = nx[j];
-        } else {
-            tile_outer<4>(it, dt, t >> 3, (t & 7) * 8, p.gw1);
+            for (int i = 0; i < 4; ++i) {
+                atomicAdd(gw + i * mlp::kH, acc[i][0].x);
+                atomicAdd(gw + i * mlp::kH + 1, acc[i][0].y);
+                atomicAdd(gw + i * mlp::kH + 2, acc[i][1].x);
+                atomicAdd(gw + i * mlp::kH + 3, acc[i][1].y);
+            }
+        }
+        // da_{l-1}: rows 8 g0 .. 8 g0 + 7, columns c0 .. c0 + 3
+        const float *wt = layer == 3 ? wt3 : wt2;
+        float2 acc[8][2];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = make_float2(0.f, 0.f);
+#pragma unroll 2
+        for (int k = 0; k < mlp::kH; k += 4) {
+            float4 w[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) w[q] = *reinterpret_cast<const float4 *>(wt + (k + q) * mlp::kH + c0);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float4 d = *reinterpret_cast<const float4 *>(dt + (8 * g0 + j) * kTileStride + k);
+                fma4(acc[j], d.x, w[0]);
+                fma4(acc[j], d.y, w[1]);
+                fma4(acc[j], d.z, w[2]);
+                fma4(acc[j], d.w, w[3]);
+            }
+        }
+        __syncthreads();  // every thread has read da
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int r = 8 * g0 + j;
+            const float4 h = *reinterpret_cast<const float4 *>(it + r * kTileStride + c0);
+            *reinterpret_cast<float4 *>(dt + r * kTileStride + c0) =
+                make_float4(h.x > 0.0f ? acc[j][0].x : 0.0f, h.y > 0.0f ? acc[j][0].y : 0.0f,
+                            h.z > 0.0f ? acc[j][1].x : 0.0f, h.w > 0.0f ? acc[j][1].y : 0.0f);
         }
     }
 }
@@ -1071,17 +1190,21 @@ __global__ void k_batch_rows(int32_t *rows, int n, uint32_t pixels, uint32_t off
     rows[r] = (int32_t)(((uint64_t)r * stride + offset) % pixels);
 }
 
-template <int kMode>
-constexpr int fused_smem() {
-    return (kMode == kGrad ? kSmemGrad : kSmemUsed) < kSmemMin ? kSmemMin : (kMode == kGrad ? kSmemGrad : kSmemUsed);
+__global__ void k_check_rows(const int32_t *rows, const int32_t *targets, int n, int64_t pixels, int c, uint32_t *bad) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    if (rows[r] < 0 || rows[r] >= pixels) atomicMin(bad, (uint32_t)r);
+    if (targets[r] < -1 || targets[r] >= c) atomicMin(bad + 1, (uint32_t)r);
 }
+
+constexpr int kFusedSmem = kSmemUsed < kSmemMin ? kSmemMin : kSmemUsed;
 
 // set_attr: set the shared-memory attribute first (the batched launches set it
 // once, before any stream capture, in prepare_views)
 template <int kMode, bool kViews = false>
 cudaError_t launch_fused(const FusedParams &p, cudaStream_t st, bool set_attr = true) {
     if (p.pd.c % kChunkN != 0 || p.pd.c < kChunkN) return cudaErrorInvalidValue;
-    constexpr int smem = fused_smem<kMode>();
+    constexpr int smem = kFusedSmem;
     if (set_attr) {
         cudaError_t e =
             cudaFuncSetAttribute(k_mlp_fused<kMode, kViews>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1121,10 +1244,10 @@ cudaError_t forward_sample(const ProposalDev &pd, const GBufView &g, const float
 
 cudaError_t prepare_views() {
     cudaError_t e = cudaFuncSetAttribute(k_mlp_fused<kLse, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         fused_smem<kLse>());
+                                         kFusedSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_mlp_fused<kSample, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 fused_smem<kSample>());
+                                 kFusedSmem);
     return e;
 }
 
@@ -1146,14 +1269,14 @@ cudaError_t forward_sample_views(const ProposalDev &pd, const ViewRows *views, i
     return launch_fused<kSample, true>(p, st, false);
 }
 
-cudaError_t forward_grad(const ProposalDev &pd, const GBufView &g, const float cam[3], const int32_t *rows, int n,
-                         const float4 *stat, const int32_t *target, float inv_n, float *dh3, float *loss_sum,
-                         int *err, cudaStream_t st) {
-    FusedParams p{};
-    p.pd = pd; p.g = g; p.cam[0] = cam[0]; p.cam[1] = cam[1]; p.cam[2] = cam[2];
-    p.rows = rows; p.n = n; p.stat = const_cast<float4 *>(stat); p.target = target; p.inv_n = inv_n; p.dh3 = dh3;
-    p.loss_sum = loss_sum; p.err = err;
-    return launch_fused<kGrad>(p, st);
+cudaError_t forward_grad(const ProposalDev &pd, const __nv_bfloat16 *h3, int n, const float4 *stat,
+                         const int32_t *target, float inv_n, float *dh3, float *loss_sum, int *err, cudaStream_t st) {
+    const GradParams p{pd, h3, stat, target, n, inv_n, dh3, loss_sum, err};
+    if (pd.c % kChunkN != 0 || pd.c < kChunkN) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem);
+    if (e != cudaSuccess) return e;
+    if (n > 0) k_mlp_grad<<<(n + kRows - 1) / kRows, kRows, kGradSmem, st>>>(p);
+    return cudaGetLastError();
 }
 
 cudaError_t dw4(const ProposalDev &pd, const __nv_bfloat16 *h3, const float4 *stat, const int32_t *target, int n,
@@ -1162,8 +1285,12 @@ cudaError_t dw4(const ProposalDev &pd, const __nv_bfloat16 *h3, const float4 *st
     Dw4Params p{pd, h3, stat, target, n, 0, inv_n, gw4, gb4, err};
     const int tiles = (n + kRows - 1) / kRows;
     const int chunks = pd.c / kChunkN;
-    // about RG_DW4_SLICE_CTAS CTAs per SM in all; each keeps its tiles' sum in tensor memory
-    int slices = (RG_DW4_SLICE_CTAS * 152 + chunks - 1) / chunks;
+    // as many slices as keep every CTA resident at once (three per SM by shared
+    // memory): 640 CTAs ran as one full round and one of 184 (65,536 rows, 4096
+    // clusters: 0.335 ms; one round, with the next rows loaded under this tile's
+    // work and the one-hot in its own piece only: 0.289)
+    int slices = 3 * 152 / chunks;
+    if (slices < 1) slices = 1;
     if (slices > tiles) slices = tiles;
     p.tiles_per_slice = (tiles + slices - 1) / slices;
     slices = (tiles + p.tiles_per_slice - 1) / p.tiles_per_slice;
@@ -1178,7 +1305,7 @@ cudaError_t backward_rows(const __nv_bfloat16 *w123, const TrainBuffers &t, cons
     BackParams p{w123, t.x, t.h1, t.h2, t.h3, dh3, gw1, gw2, gw3, gb1, gb2, gb3, n};
     cudaError_t e = cudaFuncSetAttribute(k_mlp_backward_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, kBackSmem);
     if (e != cudaSuccess) return e;
-    if (n > 0) k_mlp_backward_rows<<<(n + 127) / 128, 128, kBackSmem, st>>>(p);
+    if (n > 0) k_mlp_backward_rows<<<(n + 127) / 128, kBackThreads, kBackSmem, st>>>(p);
     return cudaGetLastError();
 }
 
@@ -1201,6 +1328,12 @@ cudaError_t refresh(const float *params, int c, const uint8_t *valid, __nv_bfloa
 cudaError_t targets(const rg_reservoir *res, const int32_t *rows, int n, const int32_t *cluster_of, int n_lights,
                     int32_t *target, int *count, cudaStream_t st) {
     if (n > 0) k_targets<<<(n + 127) / 128, 128, 0, st>>>(res, rows, n, cluster_of, n_lights, target, count);
+    return cudaGetLastError();
+}
+
+cudaError_t check_rows(const int32_t *rows, const int32_t *targets, int n, int64_t pixels, int c, uint32_t *bad,
+                       cudaStream_t st) {
+    if (n > 0) k_check_rows<<<(n + 127) / 128, 128, 0, st>>>(rows, targets, n, pixels, c, bad);
     return cudaGetLastError();
 }
 

@@ -126,9 +126,8 @@ cudaError_t forward_lse_views(const ProposalDev &pd, const ViewRows *views, int 
                               int total, float4 *stat, Candidate *cand, int *err, cudaStream_t st);
 cudaError_t forward_sample_views(const ProposalDev &pd, const ViewRows *views, int n_views, const uint32_t *frames,
                                  int total, const float4 *stat, Candidate *cand, int *err, cudaStream_t st);
-cudaError_t forward_grad(const ProposalDev &pd, const GBufView &g, const float cam[3], const int32_t *rows, int n,
-                         const float4 *stat, const int32_t *target, float inv_n, float *dh3, float *loss_sum,
-                         int *err, cudaStream_t st);
+cudaError_t forward_grad(const ProposalDev &pd, const __nv_bfloat16 *h3, int n, const float4 *stat,
+                         const int32_t *target, float inv_n, float *dh3, float *loss_sum, int *err, cudaStream_t st);
 // Adds dW4 (64 x C) and db4 of the mean loss to gw4 / gb4.
 cudaError_t dw4(const ProposalDev &pd, const __nv_bfloat16 *h3, const float4 *stat, const int32_t *target, int n,
                 float inv_n, float *gw4, float *gb4, int *err, cudaStream_t st);
@@ -141,6 +140,9 @@ cudaError_t refresh(const float *params, int c, const uint8_t *valid, __nv_bfloa
                     __nv_bfloat16 *w4k, __nv_bfloat16 *w123, __nv_bfloat16 *w4, float *b4e, cudaStream_t st);
 cudaError_t targets(const rg_reservoir *res, const int32_t *rows, int n, const int32_t *cluster_of, int n_lights,
                     int32_t *target, int *count, cudaStream_t st);
+// bad[0], bad[1] (all ones before): the first index whose row is not in [0, pixels), whose target is not in [-1, c).
+cudaError_t check_rows(const int32_t *rows, const int32_t *targets, int n, int64_t pixels, int c, uint32_t *bad,
+                       cudaStream_t st);
 cudaError_t batch_rows(int32_t *rows, int n, uint32_t pixels, uint32_t offset, uint32_t stride, cudaStream_t st);
 
 }  // namespace mlp

@@ -85,6 +85,7 @@ struct ProposalState {
     float *dh3 = nullptr;
     float *loss = nullptr;
     int *count = nullptr;
+    uint32_t *bad = nullptr;  // first bad row, first bad target of rg_proposal_gradients
     bool has_loss = false;
 
     mlp::ProposalDev dev() const {
@@ -113,7 +114,7 @@ struct ProposalState {
     void release_all() {
         release(params); release(grad); release(adam_m); release(adam_v); release(w123img); release(w4t); release(w4k);
         release(w123); release(w4); release(b4e); release(valid); release(cluster_of); release(offset); release(lcol);
-        release(within); release(stat); release(cand); release(loss); release(count);
+        release(within); release(stat); release(cand); release(loss); release(count); release(bad);
         release_train();
         inf_cap = 0;
     }
@@ -181,7 +182,7 @@ int gradients(ProposalState &ps, const GBufView &g, const float cam[3], int n, c
     PR_CUDA(cudaMemsetAsync(ps.loss, 0, sizeof(float), st), "memset");
     PR_CUDA(cudaMemsetAsync(ps.grad, 0, ps.n_params * sizeof(float), st), "memset");
     // dh3 = dz W4^T and the loss (dz stays on chip), then dW4 and db4
-    PR_CUDA(mlp::forward_grad(pd, g, cam, ps.rows, n, ps.tstat, ps.target, 1.0f / (float)n, ps.dh3, ps.loss, ps.err, st),
+    PR_CUDA(mlp::forward_grad(pd, ps.h3, n, ps.tstat, ps.target, 1.0f / (float)n, ps.dh3, ps.loss, ps.err, st),
             "proposal logits gradient");
     PR_CUDA(mlp::dw4(pd, ps.h3, ps.tstat, ps.target, n, 1.0f / (float)n, ps.grad + L.w4, ps.grad + L.b4, ps.err, st),
             "dW4");
@@ -325,6 +326,7 @@ int rg_proposal_create(rg_context *ctx, const rg_proposal_config *cfg, const rg_
     if (e == cudaSuccess) e = alloc(&ps->within, (size_t)n);
     if (e == cudaSuccess) e = alloc(&ps->loss, 1);
     if (e == cudaSuccess) e = alloc(&ps->count, 1);
+    if (e == cudaSuccess) e = alloc(&ps->bad, 2);
     if (e == cudaSuccess) e = cudaMemcpy(ps->params, params.data(), L.total * 4, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(ps->adam_m, 0, L.total * 4);
     if (e == cudaSuccess) e = cudaMemset(ps->adam_v, 0, L.total * 4);
@@ -442,19 +444,20 @@ int rg_proposal_gradients(rg_context *ctx, const rg_gbuffer *g, const float cam[
     if (rc) return rc;
     if ((rc = check_gbuf(g))) return rc;
     if (!cam || !rows || !targets || !grad || n <= 0) return pfail(RG_ERR_INVALID_ARGUMENT, "bad arguments");
-    std::vector<int32_t> hr((size_t)n), ht((size_t)n);
     cudaStream_t st = (cudaStream_t)stream;
-    PR_CUDA(cudaStreamSynchronize(st), "sync");
-    PR_CUDA(cudaMemcpy(hr.data(), rows, (size_t)n * 4, cudaMemcpyDeviceToHost), "rows");
-    PR_CUDA(cudaMemcpy(ht.data(), targets, (size_t)n * 4, cudaMemcpyDeviceToHost), "targets");
     const int64_t np = (int64_t)g->width * g->height;
-    for (int32_t i = 0; i < n; ++i) {
-        if (hr[(size_t)i] < 0 || hr[(size_t)i] >= np) return pfail(RG_ERR_INVALID_ARGUMENT, "row %d out of range", i);
-        if (ht[(size_t)i] < -1 || ht[(size_t)i] >= ps->c) return pfail(RG_ERR_INVALID_ARGUMENT, "target %d out of range", i);
-    }
     if ((rc = ensure_train(*ps, n))) return rc;
     PR_CUDA(cudaMemcpyAsync(ps->rows, rows, (size_t)n * 4, cudaMemcpyDeviceToDevice, st), "rows");
     PR_CUDA(cudaMemcpyAsync(ps->target, targets, (size_t)n * 4, cudaMemcpyDeviceToDevice, st), "targets");
+    // the first bad row or target, found on the device from these copies
+    uint32_t bad[2];
+    PR_CUDA(cudaMemsetAsync(ps->bad, 0xff, sizeof(bad), st), "rows");
+    PR_CUDA(mlp::check_rows(ps->rows, ps->target, n, np, ps->c, ps->bad, st), "rows");
+    PR_CUDA(cudaMemcpyAsync(bad, ps->bad, sizeof(bad), cudaMemcpyDeviceToHost, st), "rows");
+    PR_CUDA(cudaStreamSynchronize(st), "sync");
+    if (bad[0] != 0xffffffffu && bad[0] <= bad[1])
+        return pfail(RG_ERR_INVALID_ARGUMENT, "row %d out of range", (int)bad[0]);
+    if (bad[1] != 0xffffffffu) return pfail(RG_ERR_INVALID_ARGUMENT, "target %d out of range", (int)bad[1]);
     if ((rc = gradients(*ps, make_view(g), cam, n, st))) return rc;
     PR_CUDA(cudaMemcpyAsync(grad, ps->grad, ps->n_params * 4, cudaMemcpyDeviceToDevice, st), "grad");
     if (loss_sum) {
