@@ -56,6 +56,7 @@ constexpr int kChunkBytes = kChunkN * mlp::kH * 2;
 constexpr int kOffBias = kOffB + 2 * kChunkBytes;      // b1 | b2 | b3
 constexpr int kSmemUsed = kOffBias + 3 * mlp::kH * 4;
 constexpr int kWkBytes = mlp::kH * kChunkN * 2;
+constexpr int kHTileBytes = kRows * mlp::kH * 2;       // 128 rows of a saved hidden layer, laid out as the MMA operand tile
 constexpr int kSmemMin = 52 * 1024;                    // caps residency at four CTAs per SM (TMEM: 4 x 128 columns)
 constexpr int kWeightImgBytes = (mlp::kH * mlp::kIn + 2 * mlp::kH * mlp::kH) * 2;
 
@@ -163,7 +164,7 @@ struct FusedParams {
     float4 *stat;              // per row: lse, arg-max cluster (int bits), its probability, 0
     // training (kLse with save != 0)
     int save;
-    __nv_bfloat16 *x, *h1, *h2, *h3;  // [n x 16], [n x 64] x 3
+    __nv_bfloat16 *x, *h1, *h2, *h3;  // [n x 16]; the hidden layers by tiles of 128 rows (zeros from row n on)
     // sampling
     mlp::Candidate *cand;      // [n x kCand]
     uint32_t frame;
@@ -213,9 +214,9 @@ __device__ __forceinline__ void store8(__nv_bfloat16 *dst, const float *v) {
 
 // One 32-column piece of a row's logit gradient, (softmax - onehot) / n as
 // bf16 into the K-major dz tile: v holds the logits, nl2 = -lse * log2(e),
-// hit = target - first column or kNoTarget (the row's gradient is 0).  Only the piece that holds a row's target pays for the one-hot:
-// testing every column took 445 instructions a piece instead of about 150.
-// Returns the target's logit where the piece holds it, else 0.
+// hit = target - first column or kNoTarget (the row's gradient is 0).  Only the
+// piece that holds a row's target pays for the one-hot: testing every column
+// took 445 instructions a piece instead of about 150.  Returns the target's logit where the piece holds it, else 0.
 constexpr int kNoTarget = INT32_MIN;
 __device__ __forceinline__ float grad_piece(unsigned char *dztile, int row, int col0, const float2 (&v)[16], float nl2,
                                             float inv_n, int hit) {
@@ -225,17 +226,6 @@ __device__ __forceinline__ float grad_piece(unsigned char *dztile, int row, int 
     for (int k = 0; k < 16; ++k) {
         const float2 t = __ffma2_rn(v[k], l2, o2);
         d[k] = __fmul2_rn(make_float2(ex2(t.x), ex2(t.y)), s2);
-    }
-    float zt = 0.0f;
-    if ((unsigned)hit < 32u) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-            if (i == hit) {
-                zt = col(v, i);
-                const float g = (ex2(__fmaf_rn(zt, kLog2e, nl2)) - 1.0f) * inv_n;
-                if (i & 1) d[i >> 1].y = g;
-                else d[i >> 1].x = g;
-            }
     }
     if (hit == kNoTarget) {
 #pragma unroll
@@ -251,6 +241,20 @@ __device__ __forceinline__ float grad_piece(unsigned char *dztile, int row, int 
             b[k] = *reinterpret_cast<const uint32_t *>(&h);
         }
         *reinterpret_cast<uint4 *>(dztile + umma::kmajor_offset(row, col0 + q, kChunkN)) = w;
+    }
+    float zt = 0.0f;
+    if ((unsigned)hit < 32u) {  // the one-hot column: its logit by five rounds of selects, its gradient over the one stored
+        float2 t[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t[k] = (hit & 16) ? v[k + 8] : v[k];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) t[k] = (hit & 8) ? t[k + 4] : t[k];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) t[k] = (hit & 4) ? t[k + 2] : t[k];
+        t[0] = (hit & 2) ? t[1] : t[0];
+        zt = (hit & 1) ? t[0].y : t[0].x;
+        *reinterpret_cast<__nv_bfloat16 *>(dztile + umma::kmajor_offset(row, col0 + hit, kChunkN)) =
+            __float2bfloat16_rn((ex2(__fmaf_rn(zt, kLog2e, nl2)) - 1.0f) * inv_n);
     }
     return zt;
 }
@@ -390,9 +394,12 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
             for (int j = 0; j < 64; ++j) v[j] = bf16r(fmaxf(v[j] + bias[64 * l + j], 0.0f));
 #pragma unroll
             for (int j = 0; j < 64; j += 8) put8(htile, tid, j, mlp::kH, v + j);
-            if (kMode == kLse && p.save && valid) {
+            if (kMode == kLse && p.save) {  // as the tile itself: eight rows' 16 bytes are one 128-byte line
+                unsigned char *dst = reinterpret_cast<unsigned char *>(hsave[l]) + (size_t)blockIdx.x * kHTileBytes;
 #pragma unroll
-                for (int j = 0; j < 64; j += 8) store8(hsave[l] + (size_t)row * mlp::kH + j, v + j);
+                for (int j = 0; j < 64; ++j) v[j] = valid ? v[j] : 0.0f;
+#pragma unroll
+                for (int j = 0; j < 64; j += 8) put8(dst, tid, j, mlp::kH, v + j);
             }
         }
         umma::fence_proxy_async();
@@ -636,7 +643,7 @@ constexpr int kGradTmem = 2 * kChunkN;                     // z, dh3
 
 struct GradParams {
     mlp::ProposalDev pd;
-    const __nv_bfloat16 *h3;   // [n x 64]
+    const __nv_bfloat16 *h3;   // by tiles of 128 rows
     const float4 *stat;        // per row: lse first
     const int32_t *target;     // cluster per row, -1: no target
     int n;
@@ -659,16 +666,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_grad(const GradParams p) {
     const unsigned char *w4kimg = reinterpret_cast<const unsigned char *>(p.pd.w4k);
     copy_bytes(btile, w4img, kChunkBytes);
     copy_bytes(wk, w4kimg, kWkBytes);
-    // the saved h3 rows, eight threads a row
-    for (int e = tid; e < kRows * 8; e += kRows) {
-        const int r = e >> 3, j = e & 7;
-        unsigned char *dst = htile + umma::kmajor_offset(r, 8 * j, mlp::kH);
-        if (blockIdx.x * kRows + r < p.n)
-            cp_async16(dst, reinterpret_cast<const unsigned char *>(p.h3) +
-                                ((size_t)(blockIdx.x * kRows + r) * mlp::kH + 8 * j) * 2);
-        else
-            *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
-    }
+    copy_bytes(htile, reinterpret_cast<const unsigned char *>(p.h3) + (size_t)blockIdx.x * kHTileBytes, kHTileBytes);
     cp_async_commit();
     if (warp == 0) umma::tmem_alloc(&tmem_base, kGradTmem);
     if (tid == 0) {
@@ -787,16 +785,32 @@ __global__ void __launch_bounds__(128, 4) k_mlp_grad(const GradParams p) {
 // CTA adds its 65 x 64 result to the gradient with atomics at the end.
 //
 // No operand is transposed element by element: the h tile (rows x [h3 | 1 |
-// 0], K-major over its 128 columns) and the dz tile (rows x clusters, K-major
+// 0], K-major over its 72 columns) and the dz tile (rows x clusters, K-major
 // over clusters) are read a second time through MN-major descriptors, as
-// [h3 | 1 | 0]^T (M = 128 columns, K = rows) and dz^T (N = clusters, K =
-// rows): in the canonical no-swizzle layouts a core matrix is 8 rows of 16
-// bytes either way, with SBO the step between core matrices along M/N and
-// LBO the step along K.  The tiles sit at the start of a 64 KB allocation, so
-// every address those descriptors can form stays inside it.
+// [h3 | 1 | 0]^T (M, K = rows) and dz^T (N = clusters, K = rows): in the
+// canonical no-swizzle layouts a core matrix is 8 rows of 16 bytes either way,
+// with SBO the step between core matrices along M/N and LBO the step along K.
+// M is 128, so columns 72..127 of that operand are the next row groups' (past
+// the last one, the bytes behind the tile): they only reach product rows 72 to
+// 127, which nothing reads.
+//
+// Bound by the latency of a tile's chain (products, logits out, dz in) at
+// three CTAs an SM, so the next tile's logits are issued behind this tile's
+// product after the one barrier, from a second h tile, and that tile travels
+// in registers meanwhile.  h3 comes in the tile's own layout: rows of a plain
+// matrix cost 33 cycles of the load pipe per instruction, and their transposed
+// stores conflict.  65,536 rows x 4096 clusters: 0.289 ms with one h tile, two
+// barriers and plain rows; 0.248 with the second tile; 0.158 with the layout
+// and the biases in shared memory.  256 threads and two CTAs an SM: 0.20.
+// dst[0..3] += v[0..3], dst on a 16-byte boundary
+__device__ __forceinline__ void red_add4(float *dst, const float *v) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+                 : "memory");
+}
+
 struct Dw4Params {
     mlp::ProposalDev pd;
-    const __nv_bfloat16 *h3;   // [n x 64]
+    const __nv_bfloat16 *h3;   // by tiles of 128 rows
     const float4 *stat;        // lse per row
     const int32_t *target;
     int n, tiles_per_slice;
@@ -805,21 +819,24 @@ struct Dw4Params {
     int *err;
 };
 
-constexpr int kDwHCols = 128;                                // h tile columns: h3 (64) | 1 | 0 ... 0
-constexpr int kDwOffH = 0;                                   // h tile, 128 rows x 128 (K-major, 32 KB)
-constexpr int kDwOffDz = kDwOffH + kRows * kDwHCols * 2;     // dz tile, 128 rows x 64 (K-major, 16 KB)
+constexpr int kDwHCols = 72;                                 // h tile columns: h3 (64) | 1 | 0 ... 0
+constexpr int kDwHBytes = kRows * kDwHCols * 2;
+constexpr int kDwOffH = 0;                                   // two h tiles, 128 rows x 72 (K-major, 18 KB each)
+constexpr int kDwOffDz = kDwOffH + 2 * kDwHBytes;            // dz tile, 128 rows x 64 (K-major, 16 KB)
 constexpr int kDwOffBz = kDwOffDz + kRows * kChunkN * 2;     // W4^T chunk, 64 x 64 (K-major, 8 KB)
-constexpr int kDwSmem = 64 * 1024;
+constexpr int kDwSmem = kDwOffBz + kChunkBytes;
+constexpr int kDwCtas = 3;                                   // resident per SM (shared memory, registers)
 
 // kind::f16 instruction descriptor with both operands MN-major (bits 15, 16)
 __device__ __forceinline__ uint32_t idesc_mn_major(int m, int n) {
     return umma::idesc_bf16_f32(m, n) | (1u << 15) | (1u << 16);
 }
 
-__global__ void __launch_bounds__(128, 3) k_mlp_dw4(const Dw4Params p) {
+__global__ void __launch_bounds__(kRows, kDwCtas) k_mlp_dw4(const Dw4Params p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint64_t mbar_z, mbar_w;
     __shared__ uint32_t tmem_base;
+    __shared__ __align__(16) float bias[kChunkN];
     const int tid = threadIdx.x, warp = tid >> 5;
     const int chunk = blockIdx.x;
     const int t0 = blockIdx.y * p.tiles_per_slice;
@@ -827,21 +844,50 @@ __global__ void __launch_bounds__(128, 3) k_mlp_dw4(const Dw4Params p) {
     unsigned char *ht = smem + kDwOffH, *dzt = smem + kDwOffDz, *bz = smem + kDwOffBz;
     copy_bytes(bz, reinterpret_cast<const unsigned char *>(p.pd.w4t) + (size_t)chunk * kChunkBytes, kChunkBytes);
     cp_async_commit();
-    {  // this thread's row of the h tile, columns 64..127: 1 (the db4 row of the product), then zeros
+    for (int r = tid; r < 2 * kRows; r += kRows) {  // columns 64..71 of both tiles: 1 (the db4 row of the product), zeros
         __align__(16) __nv_bfloat16 one[8];
         one[0] = __float2bfloat16_rn(1.0f);
 #pragma unroll
         for (int i = 1; i < 8; ++i) one[i] = __float2bfloat16_rn(0.0f);
-        *reinterpret_cast<uint4 *>(ht + umma::kmajor_offset(tid, 64, kDwHCols)) = *reinterpret_cast<const uint4 *>(one);
-#pragma unroll
-        for (int j = 72; j < kDwHCols; j += 8)
-            *reinterpret_cast<uint4 *>(ht + umma::kmajor_offset(tid, j, kDwHCols)) = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4 *>(ht + (r / kRows) * kDwHBytes + umma::kmajor_offset(r % kRows, 64, kDwHCols)) =
+            *reinterpret_cast<const uint4 *>(one);
     }
+    if (tid < kChunkN) bias[tid] = __ldg(p.pd.b4e + chunk * kChunkN + tid);
     if (warp == 0) umma::tmem_alloc(&tmem_base, 128);
     if (tid == 0) {
         umma::mbar_init(&mbar_z, 1);
         umma::mbar_init(&mbar_w, 1);
     }
+    // a saved tile travels in registers under the work on the tile before it
+    constexpr int kPer = kHTileBytes / 16 / kRows;
+    uint4 hrow[kPer];
+    auto fetch_tile = [&](int t) {
+        if (t >= t1) return;
+        const uint4 *src = reinterpret_cast<const uint4 *>(p.h3) + (size_t)t * (kHTileBytes / 16);
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) hrow[i] = __ldg(src + i * kRows + tid);
+    };
+    auto put_tile = [&](int buf) {  // 64 pieces of 16 bytes a row group, then the group's columns 64..71
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const int q = i * kRows + tid;
+            *reinterpret_cast<uint4 *>(ht + buf * kDwHBytes + (q >> 6) * (8 * kDwHCols * 2) + (q & 63) * 16) = hrow[i];
+        }
+    };
+    float lse = 0.0f;   // of this thread's row of the next tile
+    int target = -1;
+    auto fetch_stat = [&](int t) {
+        const int row = t * kRows + tid;
+        const bool valid = t < t1 && row < p.n;
+        target = valid ? __ldg(p.target + row) : -1;
+        lse = valid ? __ldg(reinterpret_cast<const float *>(p.stat + row)) : 0.0f;
+    };
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) hrow[i] = make_uint4(0, 0, 0, 0);
+    fetch_tile(t0);
+    fetch_stat(t0);
+    put_tile(0);
+    fetch_tile(t0 + 1);
     cp_async_wait_all();
     umma::fence_proxy_async();
     umma::fence_before_sync();
@@ -851,51 +897,25 @@ __global__ void __launch_bounds__(128, 3) k_mlp_dw4(const Dw4Params p) {
     bool ok = t0 < t1, ok_warp = true;
     uint64_t *last_mbar = nullptr;
     uint32_t last_parity = 0;
-    const float4 *be = reinterpret_cast<const float4 *>(p.pd.b4e + chunk * kChunkN);
+    const float4 *be = reinterpret_cast<const float4 *>(bias);
     const uint32_t ht_a = umma::smem_addr(ht), dz_a = umma::smem_addr(dzt), bz_a = umma::smem_addr(bz);
-    // the next tile's rows travel in registers under this tile's work
-    uint4 hrow[8];  // 16 bytes of rows tid / 8 + 16 j, eight threads a row
-    auto fetch_row = [&](int t) {
+    // z = h3 . W4[:, chunk]: A = h tile (K-major, first 64 columns), B = W4^T chunk
+    auto issue_z = [&](int k) {
+        const uint32_t idesc = umma::idesc_bf16_f32(kRows, kChunkN), a = ht_a + (uint32_t)((k & 1) * kDwHBytes);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int row = t * kRows + (tid >> 3) + 16 * j;
-            hrow[j] = t < t1 && row < p.n
-                          ? __ldg(reinterpret_cast<const uint4 *>(p.h3 + (size_t)row * mlp::kH + 8 * (tid & 7)))
-                          : make_uint4(0, 0, 0, 0);
-        }
+        for (int ks = 0; ks < mlp::kH / 16; ++ks)
+            umma::mma_bf16(tmem, umma::smem_desc(a + (uint32_t)ks * 256u, 128u, (kDwHCols / 8) * 128u),
+                           umma::smem_desc(bz_a + (uint32_t)ks * 256u, 128u, (mlp::kH / 8) * 128u), idesc, ks > 0);
+        umma::mma_commit(&mbar_z);
+        last_mbar = &mbar_z;
+        last_parity = (uint32_t)(k & 1);
     };
-    if (ok) fetch_row(t0);
+    if (ok && tid == 0) issue_z(0);
     for (int t = t0; t < t1 && ok; ++t) {
         const int k = t - t0;
-        const int row = t * kRows + tid;
-        const bool valid = row < p.n;
-        float lse = 0.0f;
-        int target = -1;
-        if (valid) {
-            target = p.target[row];
-            lse = p.stat[row].x;
-        }
         const float nl2 = -lse * kLog2e;
-        if (k > 0) ok_warp = ok_warp && mma_wait(&mbar_w, (uint32_t)((k - 1) & 1));  // previous tile's operands free
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<uint4 *>(ht + umma::kmajor_offset((tid >> 3) + 16 * j, 8 * (tid & 7), kDwHCols)) = hrow[j];
-        umma::fence_proxy_async();
-        umma::fence_before_sync();
-        ok = __syncthreads_and(ok_warp) != 0;
-        umma::fence_after_sync();
-        if (!ok) break;
-        if (tid == 0) {  // z = h3 . W4[:, chunk]: A = h tile (K-major, first 64 columns), B = W4^T chunk
-            const uint32_t idesc = umma::idesc_bf16_f32(kRows, kChunkN);
-#pragma unroll
-            for (int ks = 0; ks < mlp::kH / 16; ++ks)
-                umma::mma_bf16(tmem, umma::smem_desc(ht_a + (uint32_t)ks * 256u, 128u, (kDwHCols / 8) * 128u),
-                               umma::smem_desc(bz_a + (uint32_t)ks * 256u, 128u, (mlp::kH / 8) * 128u), idesc, ks > 0);
-            umma::mma_commit(&mbar_z);
-            last_mbar = &mbar_z;
-            last_parity = (uint32_t)(k & 1);
-        }
-        fetch_row(t + 1);
+        const int hit = target < 0 ? kNoTarget : target - chunk * kChunkN;
+        fetch_stat(t + 1);
         const bool w = mma_wait(&mbar_z, (uint32_t)(k & 1));
         ok_warp = ok_warp && w;
         if (w) {
@@ -907,14 +927,19 @@ __global__ void __launch_bounds__(128, 3) k_mlp_dw4(const Dw4Params p) {
                 float2 v[16];
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    const float4 b = __ldg(be + piece * 8 + q);
+                    const float4 b = be[piece * 8 + q];
                     v[2 * q] = __fadd2_rn(make_float2(__uint_as_float(raw[4 * q]), __uint_as_float(raw[4 * q + 1])),
                                           make_float2(b.x, b.y));
                     v[2 * q + 1] = __fadd2_rn(
                         make_float2(__uint_as_float(raw[4 * q + 2]), __uint_as_float(raw[4 * q + 3])), make_float2(b.z, b.w));
                 }
+                if (piece == 0) {  // the previous product has read the dz tile and the other h tile
+                    if (k > 0) ok_warp = mma_wait(&mbar_w, (uint32_t)((k - 1) & 1)) && ok_warp;
+                    put_tile((k + 1) & 1);
+                    fetch_tile(t + 2);
+                }
                 grad_piece(dzt, tid, piece * 32, v, nl2, p.inv_n,
-                           target < 0 ? kNoTarget : target - (chunk * kChunkN + piece * 32));
+                           hit == kNoTarget ? kNoTarget : hit - piece * 32);
             }
         }
         umma::fence_proxy_async();
@@ -925,19 +950,20 @@ __global__ void __launch_bounds__(128, 3) k_mlp_dw4(const Dw4Params p) {
         if (tid == 0) {
             // dW += [h3 | 1 | 0]^T dz: both tiles through MN-major descriptors,
             // K = the tile's rows in steps of 16 (two core matrices along K)
-            const uint32_t idesc = idesc_mn_major(128, kChunkN);
+            const uint32_t idesc = idesc_mn_major(128, kChunkN), a = ht_a + (uint32_t)((k & 1) * kDwHBytes);
             constexpr uint32_t lbo_h = 8 * kDwHCols * 2, lbo_dz = 8 * kChunkN * 2;  // K step: 8 rows of a tile
 #pragma unroll
             for (int ks = 0; ks < kRows / 16; ++ks)
-                umma::mma_bf16(tmem + 64, umma::smem_desc(ht_a + (uint32_t)ks * 2u * lbo_h, lbo_h, 128u),
+                umma::mma_bf16(tmem + 64, umma::smem_desc(a + (uint32_t)ks * 2u * lbo_h, lbo_h, 128u),
                                umma::smem_desc(dz_a + (uint32_t)ks * 2u * lbo_dz, lbo_dz, 128u), idesc,
                                k > 0 || ks > 0);
             umma::mma_commit(&mbar_w);
             last_mbar = &mbar_w;
             last_parity = (uint32_t)(k & 1);
+            if (t + 1 < t1) issue_z(k + 1);
         }
     }
-    if (ok && t1 > t0) ok_warp = ok_warp && mma_wait(&mbar_w, (uint32_t)((t1 - t0 - 1) & 1));
+    if (ok && t1 > t0) ok_warp = mma_wait(&mbar_w, (uint32_t)((t1 - t0 - 1) & 1)) && ok_warp;
     ok = __syncthreads_and(ok && ok_warp) != 0;
     if (!ok && t1 > t0) {
         if (tid == 0) {
@@ -955,7 +981,7 @@ __global__ void __launch_bounds__(128, 3) k_mlp_dw4(const Dw4Params p) {
                 float *dst = m < 64 ? p.gw4 + (size_t)m * p.pd.c + chunk * kChunkN + piece * 32
                                     : p.gb4 + chunk * kChunkN + piece * 32;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) atomicAdd(dst + i, v[i]);
+                for (int i = 0; i < 32; i += 4) red_add4(dst + i, v + i);
             }
         }
     }
@@ -1002,6 +1028,20 @@ __device__ __forceinline__ void load_tile(float *tile, const __nv_bfloat16 *src,
     }
 }
 
+// The same for a saved hidden layer (128 rows laid out as the MMA operand tile).
+__device__ __forceinline__ void load_h_tile(float *tile, const __nv_bfloat16 *src) {
+    const uint4 *img = reinterpret_cast<const uint4 *>(src) + (size_t)blockIdx.x * (kHTileBytes / 16);
+    for (int e = threadIdx.x; e < kHTileBytes / 16; e += kBackThreads) {
+        const uint4 w = __ldg(img + e);
+        const __nv_bfloat162 *b = reinterpret_cast<const __nv_bfloat162 *>(&w);
+        float4 *d = reinterpret_cast<float4 *>(tile + ((e >> 6) * 8 + (e & 7)) * kTileStride + ((e >> 3) & 7) * 8);
+        const float2 f0 = __bfloat1622float2(b[0]), f1 = __bfloat1622float2(b[1]), f2 = __bfloat1622float2(b[2]),
+                     f3 = __bfloat1622float2(b[3]);
+        d[0] = make_float4(f0.x, f0.y, f1.x, f1.y);
+        d[1] = make_float4(f2.x, f2.y, f3.x, f3.y);
+    }
+}
+
 // The hidden layers' backward pass for 128 rows per block: da3 = dh3
 // relu'(h3); for l = 3, 2, 1: db_l += column sums of da_l, dW_l += in_l^T da_l
 // (in_3 = h2, in_2 = h1, in_1 = x), and da_{l-1} = (W_l da_l) relu'(h_{l-1}),
@@ -1023,7 +1063,7 @@ __global__ void __launch_bounds__(kBackThreads, 2) k_mlp_backward_rows(const Bac
         const int i = f / mlp::kH, k = f % mlp::kH;  // W[i][k]
         (layer ? wt3 : wt2)[k * mlp::kH + i] = __bfloat162float(p.w123[mlp::kIn * mlp::kH + e]);
     }
-    load_tile<mlp::kH>(it, p.h3, row0, p.n);
+    load_h_tile(it, p.h3);
     __syncthreads();
     for (int e = t; e < 128 * 16; e += kBackThreads) {  // da3
         const int r = e >> 4, c = (e & 15) * 4;
@@ -1040,8 +1080,8 @@ __global__ void __launch_bounds__(kBackThreads, 2) k_mlp_backward_rows(const Bac
 #pragma unroll 1
     for (int layer = 3; layer >= 1; --layer) {
         __syncthreads();  // da is complete and the input tile no longer read
-        if (layer == 3) load_tile<mlp::kH>(it, p.h2, row0, p.n);
-        else if (layer == 2) load_tile<mlp::kH>(it, p.h1, row0, p.n);
+        if (layer == 3) load_h_tile(it, p.h2);
+        else if (layer == 2) load_h_tile(it, p.h1);
         else load_tile<mlp::kIn>(it, p.x, row0, p.n);
         __syncthreads();
         if (t < 128) {  // db_l: thread t sums half the rows of column t % 64
@@ -1285,18 +1325,16 @@ cudaError_t dw4(const ProposalDev &pd, const __nv_bfloat16 *h3, const float4 *st
     Dw4Params p{pd, h3, stat, target, n, 0, inv_n, gw4, gb4, err};
     const int tiles = (n + kRows - 1) / kRows;
     const int chunks = pd.c / kChunkN;
-    // as many slices as keep every CTA resident at once (three per SM by shared
-    // memory): 640 CTAs ran as one full round and one of 184 (65,536 rows, 4096
-    // clusters: 0.335 ms; one round, with the next rows loaded under this tile's
-    // work and the one-hot in its own piece only: 0.289)
-    int slices = 3 * 152 / chunks;
+    // as many slices as keep every CTA resident at once: a second round of a few
+    // CTAs costs as much as a full one
+    int slices = kDwCtas * 152 / chunks;
     if (slices < 1) slices = 1;
     if (slices > tiles) slices = tiles;
     p.tiles_per_slice = (tiles + slices - 1) / slices;
     slices = (tiles + p.tiles_per_slice - 1) / p.tiles_per_slice;
     cudaError_t e = cudaFuncSetAttribute(k_mlp_dw4, cudaFuncAttributeMaxDynamicSharedMemorySize, kDwSmem);
     if (e != cudaSuccess) return e;
-    k_mlp_dw4<<<dim3(chunks, slices), 128, kDwSmem, st>>>(p);
+    k_mlp_dw4<<<dim3(chunks, slices), kRows, kDwSmem, st>>>(p);
     return cudaGetLastError();
 }
 

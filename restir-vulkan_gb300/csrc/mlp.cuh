@@ -96,7 +96,9 @@ struct LearnedRis {
     float uniform_pdf;              // (1 - mix) / N
 };
 
-// Activations of the training rows, saved by the forward pass (bf16 values).
+// Activations of the training rows, saved by the forward pass (bf16 values):
+// x by rows of 16; h1, h2, h3 by whole tiles of 128 rows laid out as the MMA
+// operand tile (umma::kmajor_offset), zeros from the last row on.
 struct TrainBuffers {
     __nv_bfloat16 *x, *h1, *h2, *h3;
 };

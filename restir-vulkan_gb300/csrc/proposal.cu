@@ -147,13 +147,14 @@ int ensure_train(ProposalState &ps, int n) {
     if (n <= ps.train_cap) return RG_OK;
     ps.release_train();
     const size_t nn = (size_t)n;
+    const size_t tiled = (nn + 127) / 128 * 128 * mlp::kH;  // saved by whole tiles of 128 rows
     cudaError_t e = alloc(&ps.rows, nn);
     if (e == cudaSuccess) e = alloc(&ps.target, nn);
     if (e == cudaSuccess) e = alloc(&ps.tstat, nn);
     if (e == cudaSuccess) e = alloc(&ps.x, nn * mlp::kIn);
-    if (e == cudaSuccess) e = alloc(&ps.h1, nn * mlp::kH);
-    if (e == cudaSuccess) e = alloc(&ps.h2, nn * mlp::kH);
-    if (e == cudaSuccess) e = alloc(&ps.h3, nn * mlp::kH);
+    if (e == cudaSuccess) e = alloc(&ps.h1, tiled);
+    if (e == cudaSuccess) e = alloc(&ps.h2, tiled);
+    if (e == cudaSuccess) e = alloc(&ps.h3, tiled);
     if (e == cudaSuccess) e = alloc(&ps.dh3, nn * mlp::kH);
     if (e != cudaSuccess) {
         ps.release_train();
