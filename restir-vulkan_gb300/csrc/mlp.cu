@@ -7,7 +7,13 @@
 // memory so that the MMA of chunk c+1 runs under the epilogue of chunk c.
 // Weight tiles arrive by cp.async from bf16 images that are already in the MMA
 // operand layout.  Logits never leave the SM.  Exponentials are 2^x on the MUFU
-// unit with the log2(e) scale folded into one FMA per logit.  Two epilogues:
+// unit with the log2(e) scale folded into one FMA per logit.  Bound by issue
+// slots and by the latency of the epilogues (55-60 % of the slots, 15 warps an
+// SM), so they read b4 from shared memory (global loads, even from L1, were
+// most of the stalls), and kSample draws a row's uniforms before its search
+// and kLse finds an arg-max by triples.  2,073,600 rows and 4096 clusters,
+// both passes: 7.38 ms before these, 7.01 with the uniforms, 6.82 with the
+// biases, 6.72 with the rest.  Two epilogues:
 //   kLse     log-sum-exp, arg-max and its probability per row;
 //   kSample  the learned-branch candidates: each row walks its softmax CDF
 //            once with its uniforms drawn as ascending order statistics; a
@@ -54,7 +60,12 @@ constexpr int kOffW3 = kOffW2 + mlp::kH * mlp::kH * 2;
 constexpr int kOffB = kOffW3 + mlp::kH * mlp::kH * 2;  // two chunk tiles, 128 x 64
 constexpr int kChunkBytes = kChunkN * mlp::kH * 2;
 constexpr int kOffBias = kOffB + 2 * kChunkBytes;      // b1 | b2 | b3
+static_assert(kOffB - kOffW1 >= (mlp::kCand + 1) * kRows * 4, "kSample's uniforms lie over the hidden weights");
 constexpr int kSmemUsed = kOffBias + 3 * mlp::kH * 4;
+// b4 of three chunks, in turn, over the x tile once layer 1 has read it
+constexpr int kOffB4 = kOffX;
+constexpr int kB4Bytes = kChunkN * 4;
+static_assert(3 * kB4Bytes <= kRows * mlp::kIn * 2, "three chunks' biases fit the x tile");
 constexpr int kWkBytes = mlp::kH * kChunkN * 2;
 constexpr int kHTileBytes = kRows * mlp::kH * 2;       // 128 rows of a saved hidden layer, laid out as the MMA operand tile
 constexpr int kSmemMin = 52 * 1024;                    // caps residency at four CTAs per SM (TMEM: 4 x 128 columns)
@@ -81,13 +92,27 @@ __device__ __forceinline__ float max3f(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
     return y;
 }
-__device__ __forceinline__ float max32(const float2 (&v)[16]) {
-    float a[11];
+// The piece's maximum; a: the maxima of columns 3 k .. 3 k + 2.
+__device__ __forceinline__ float max32(const float2 (&v)[16], float (&a)[11]) {
 #pragma unroll
     for (int k = 0; k < 10; ++k) a[k] = max3f(col(v, 3 * k), col(v, 3 * k + 1), col(v, 3 * k + 2));
     a[10] = fmaxf(col(v, 30), col(v, 31));
     const float b0 = max3f(a[0], a[1], a[2]), b1 = max3f(a[3], a[4], a[5]), b2 = max3f(a[6], a[7], a[8]);
     return fmaxf(max3f(b0, b1, b2), fmaxf(a[9], a[10]));
+}
+// The first column whose value is the maximum mp, by its triple (44
+// instructions; one test per column takes 64).
+__device__ __forceinline__ int first_max(const float2 (&v)[16], const float (&a)[11], float mp) {
+    int t = 10;
+    float e0 = col(v, 30), e1 = col(v, 31);
+#pragma unroll
+    for (int k = 9; k >= 0; --k)
+        if (a[k] == mp) {
+            t = k;
+            e0 = col(v, 3 * k);
+            e1 = col(v, 3 * k + 1);
+        }
+    return 3 * t + (e0 == mp ? 0 : e1 == mp ? 1 : 2);
 }
 __device__ __forceinline__ float sum32(const float2 (&v)[16]) {
     float2 t[8];
@@ -312,6 +337,8 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
     // weights and the first two logit chunks start moving
     copy_bytes(smem + kOffW1, reinterpret_cast<const unsigned char *>(p.pd.w123img), kWeightImgBytes);
     copy_bytes(btile[0], w4img, kChunkBytes);
+    unsigned char *b4s = smem + kOffB4;
+    const unsigned char *b4img = reinterpret_cast<const unsigned char *>(p.pd.b4e);
     cp_async_commit();
     if (nch > 1) copy_bytes(btile[1], w4img + kChunkBytes, kChunkBytes);
     cp_async_commit();
@@ -346,8 +373,6 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
     // stream (two draws per slot: branch, uniform light; then one per
     // learned slot).  The k-th smallest uniform goes to the k-th learned slot.
     uint32_t lmask = 0;  // learned slots not yet assigned
-    int n_u = 0, k_u = 0;
-    float u_prev = 0.0f;
     Pcg rng{};
     if (kMode == kSample && valid) {
         rng = pcg_seed((uint64_t)frame * mlp::kSeedMul + mlp::kSeedAdd, (uint64_t)px);
@@ -356,7 +381,6 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
             rand_float(rng);
             if (u0 < p.pd.mix) lmask |= 1u << j;
         }
-        n_u = __popc(lmask);
     }
 
     cp_async_wait_one();
@@ -387,6 +411,8 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
         }
         const bool w = mma_wait(&mbar_layer, (uint32_t)(l & 1));
         if (w) {
+            // the first two chunks' biases; the barriers of this loop come before their use
+            if (l == 1 && tid < min(nch, 2) * kChunkN) reinterpret_cast<float *>(b4s)[tid] = __ldg(p.pd.b4e + tid);
             float v[64];
             umma::tmem_ld32(lcol, warp, 0, *reinterpret_cast<float(*)[32]>(v));
             umma::tmem_ld32(lcol, warp, 32, *reinterpret_cast<float(*)[32]>(v + 32));
@@ -412,7 +438,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
     float m = -INFINITY, s = 0.0f;  // kLse: running max and sum
     int amax = 0;
     float lse = 0.0f, cum = 0.0f;   // kSample
-    float next_u = INFINITY;  // no uniform left (cum never exceeds it, even when it overflows)
+    float next_u = INFINITY;  // the row's next uniform; INFINITY: none left (cum never exceeds it, even when it overflows)
     int amax_row = 0;
     float qmax_row = 0.0f;
     if (kMode == kSample && valid) {
@@ -420,13 +446,9 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
         lse = st.x;
         amax_row = __float_as_int(st.y);
         qmax_row = st.z;
-        if (n_u > 0) {
-            u_prev = next_order_stat(rng, 0.0f, n_u);
-            k_u = 1;
-            next_u = u_prev;
-        }
     }
     const float nl2 = -lse * kLog2e;
+    const float *uni = reinterpret_cast<const float *>(smem + kOffW1) + tid;  // kSample: the row's uniforms
     // kSample: the learned slot of the current uniform gets cluster col with q
     auto take = [&](int col, float q) {
         if (!(q > 0.0f)) {  // rounding put the uniform on an empty column: the most probable cluster
@@ -436,13 +458,8 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
         const int slot = __ffs(lmask) - 1;
         lmask &= lmask - 1;
         p.cand[(size_t)row * mlp::kCand + slot] = mlp::Candidate{-1 - col, q};
-        if (k_u < n_u) {
-            u_prev = next_order_stat(rng, u_prev, n_u - k_u);
-            ++k_u;
-            next_u = u_prev;
-        } else {
-            next_u = INFINITY;
-        }
+        uni += kRows;
+        next_u = *uni;
     };
     if (ok && tid == 0) {
         umma::mma_chunk(tmem, htile, btile[0], mlp::kH, kRows, kChunkN, false);
@@ -450,11 +467,23 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
         last_mbar = &mbar_chunk[0];
         last_parity = 0;
     }
+    // all of a row's uniforms at once (inside the search only the rows with a
+    // uniform in the piece would draw: ten times as many warp executions),
+    // over the hidden layers' weights, whose last product has completed
+    if (kMode == kSample && ok) {
+        float *us = reinterpret_cast<float *>(smem + kOffW1) + tid;
+        const int n_u = __popc(lmask);
+        float u = 0.0f;
+        for (int k = 0; k < n_u; ++k) us[k * kRows] = u = next_order_stat(rng, u, n_u - k);
+        us[n_u * kRows] = INFINITY;
+        next_u = us[0];
+    }
     // `ok` changes only at block barriers (uniform); `ok_warp` records this
     // warp's waits and joins `ok` at the next barrier, so every warp passes
     // the same sequence of barriers whatever fails.
     bool ok_warp = true;
-    for (int c = 0; c < nch; ++c) {
+    int slot = 0;  // c % 3
+    for (int c = 0; c < nch; ++c, slot = slot == 2 ? 0 : slot + 1) {
         if (!ok) break;
         if (c + 1 < nch) {
             cp_async_wait_all();
@@ -476,6 +505,8 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
         if (w) {
         if (c + 2 < nch) {
             copy_bytes(btile[c & 1], w4img + (size_t)(c + 2) * kChunkBytes, kChunkBytes);
+            // chunk c - 1's biases, the third place, were last read before this chunk's barrier
+            copy_bytes(b4s + (slot == 0 ? 2 : slot - 1) * kB4Bytes, b4img + (size_t)(c + 2) * kB4Bytes, kB4Bytes);
             cp_async_commit();
         }
         const uint32_t half = tmem + (uint32_t)((c & 1) * kChunkN);
@@ -488,24 +519,21 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
             if (piece + 1 < kChunkN / 32) umma::tmem_ld32_issue(half, warp, (piece + 1) * 32, raw[(piece + 1) & 1]);
             const uint32_t(&rw)[32] = raw[piece & 1];
             const int col0 = c * kChunkN + piece * 32;
-            const float4 *be = reinterpret_cast<const float4 *>(p.pd.b4e + col0);
+            const float4 *be = reinterpret_cast<const float4 *>(b4s + slot * kB4Bytes) + piece * 8;
             float2 v[16];  // logits z = MMA result + b4
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                const float4 b = __ldg(be + q);
+                const float4 b = be[q];
                 v[2 * q] = __fadd2_rn(make_float2(__uint_as_float(rw[4 * q]), __uint_as_float(rw[4 * q + 1])),
                                       make_float2(b.x, b.y));
                 v[2 * q + 1] = __fadd2_rn(make_float2(__uint_as_float(rw[4 * q + 2]), __uint_as_float(rw[4 * q + 3])),
                                           make_float2(b.z, b.w));
             }
             if (kMode == kLse) {
-                const float mp = max32(v);
+                float triple[11];
+                const float mp = max32(v, triple);
                 if (mp == -INFINITY) continue;
-                if (mp > m) {
-#pragma unroll
-                    for (int i = 31; i >= 0; --i)
-                        if (col(v, i) == mp) amax = col0 + i;
-                }
+                if (mp > m) amax = col0 + first_max(v, triple, mp);
                 exp_piece(v, -mp * kLog2e);
                 const float sp = sum32(v);
                 if (mp > m) {
@@ -582,32 +610,28 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
                         h[j + 2 * i + 1] = f.y;
                     }
                 }
-                Pcg r2 = pcg_seed((uint64_t)frame * mlp::kSeedMul + mlp::kSeedAdd, (uint64_t)px);
+                rng = pcg_seed((uint64_t)frame * mlp::kSeedMul + mlp::kSeedAdd, (uint64_t)px);
                 const float nl = -lse_row * kLog2e;
                 // first the slots that take the uniform branch (about 1 in 10),
                 // then one loop iteration per such slot of this row: the warp
                 // runs as many dot products as its busiest row has slots, not
                 // one per slot index that any row uses
                 uint32_t umask = 0;
-                {
-                    Pcg r1 = r2;
-                    for (int j = 0; j < n_cand; ++j) {
-                        const float u0 = rand_float(r1);
-                        rand_float(r1);
-                        if (!(u0 < p.pd.mix)) umask |= 1u << j;
+                float *us = reinterpret_cast<float *>(smem + kOffW1) + tid;  // their draws, over the hidden weights
+                for (int j = 0; j < n_cand; ++j) {
+                    const float u0 = rand_float(rng), u1 = rand_float(rng);
+                    if (!(u0 < p.pd.mix)) {
+                        *us = u1;
+                        us += kRows;
+                        umask |= 1u << j;
                     }
                 }
-                int pos = 0;  // slots of r2's stream consumed
+                us = reinterpret_cast<float *>(smem + kOffW1) + tid;
                 while (umask) {
                     const int j = __ffs(umask) - 1;
                     umask &= umask - 1;
-                    for (; pos < j; ++pos) {
-                        rand_float(r2);
-                        rand_float(r2);
-                    }
-                    rand_float(r2);
-                    const float u1 = rand_float(r2);
-                    ++pos;
+                    const float u1 = *us;
+                    us += kRows;
                     const int l = imin((int)((float)p.pd.n_lights * u1), p.pd.n_lights - 1);
                     const float z = logit_of(p.pd, h, __ldg(p.pd.cluster_of + l));
                     p.cand[(size_t)row * mlp::kCand + j] = mlp::Candidate{l, ex2(__fmaf_rn(z, kLog2e, nl))};
