@@ -13,7 +13,8 @@
 // most of the stalls), and kSample draws a row's uniforms before its search
 // and kLse finds an arg-max by triples.  2,073,600 rows and 4096 clusters,
 // both passes: 7.38 ms before these, 7.01 with the uniforms, 6.82 with the
-// biases, 6.72 with the rest.  Two epilogues:
+// biases, 6.72 with the rest; 6.28 once no tile's address was read from a
+// pointer array in local memory (a load from L2 a chunk).  Two epilogues:
 //   kLse     log-sum-exp, arg-max and its probability per row;
 //   kSample  the learned-branch candidates: each row walks its softmax CDF
 //            once with its uniforms drawn as ascending order statistics; a
@@ -330,17 +331,18 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
     const int nch = p.pd.c / kChunkN;
     const mlp::Layout L(p.pd.c);
     unsigned char *xtile = smem + kOffX, *htile = smem + kOffH;
-    unsigned char *btile[2] = {smem + kOffB, smem + kOffB + kChunkBytes};
+    // by arithmetic: an array of pointers indexed at run time would live in local memory
+    auto btile = [&](int i) { return smem + kOffB + i * kChunkBytes; };
     float *bias = reinterpret_cast<float *>(smem + kOffBias);
     const unsigned char *w4img = reinterpret_cast<const unsigned char *>(p.pd.w4t);
 
     // weights and the first two logit chunks start moving
     copy_bytes(smem + kOffW1, reinterpret_cast<const unsigned char *>(p.pd.w123img), kWeightImgBytes);
-    copy_bytes(btile[0], w4img, kChunkBytes);
+    copy_bytes(btile(0), w4img, kChunkBytes);
     unsigned char *b4s = smem + kOffB4;
     const unsigned char *b4img = reinterpret_cast<const unsigned char *>(p.pd.b4e);
     cp_async_commit();
-    if (nch > 1) copy_bytes(btile[1], w4img + kChunkBytes, kChunkBytes);
+    if (nch > 1) copy_bytes(btile(1), w4img + kChunkBytes, kChunkBytes);
     cp_async_commit();
     for (int i = tid; i < 3 * mlp::kH; i += blockDim.x) {
         const size_t b = i < mlp::kH ? L.b1 : i < 2 * mlp::kH ? L.b2 : L.b3;
@@ -397,14 +399,12 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
     uint32_t last_parity = 0;
 
     // ---- hidden layers: MMA into columns 64*l, epilogue into the h tile
-    const unsigned char *wimg[3] = {smem + kOffW1, smem + kOffW2, smem + kOffW3};
-    __nv_bfloat16 *hsave[3] = {p.h1, p.h2, p.h3};
     for (int l = 0; l < 3 && ok; ++l) {
         // layer l accumulates in columns 64*(l&1): layer 3 reuses layer 1's,
         // whose loads completed before the barrier that preceded layer 2
         const uint32_t lcol = tmem + (uint32_t)(64 * (l & 1));
         if (tid == 0) {
-            umma::mma_chunk(lcol, l == 0 ? xtile : htile, wimg[l], l == 0 ? mlp::kIn : mlp::kH, kRows, mlp::kH, false);
+            umma::mma_chunk(lcol, l == 0 ? xtile : htile, smem + (l == 0 ? kOffW1 : l == 1 ? kOffW2 : kOffW3), l == 0 ? mlp::kIn : mlp::kH, kRows, mlp::kH, false);
             umma::mma_commit(&mbar_layer);
             last_mbar = &mbar_layer;
             last_parity = (uint32_t)(l & 1);
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
 #pragma unroll
             for (int j = 0; j < 64; j += 8) put8(htile, tid, j, mlp::kH, v + j);
             if (kMode == kLse && p.save) {  // as the tile itself: eight rows' 16 bytes are one 128-byte line
-                unsigned char *dst = reinterpret_cast<unsigned char *>(hsave[l]) + (size_t)blockIdx.x * kHTileBytes;
+                unsigned char *dst = reinterpret_cast<unsigned char *>(l == 0 ? p.h1 : l == 1 ? p.h2 : p.h3) + (size_t)blockIdx.x * kHTileBytes;
 #pragma unroll
                 for (int j = 0; j < 64; ++j) v[j] = valid ? v[j] : 0.0f;
 #pragma unroll
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
         next_u = *uni;
     };
     if (ok && tid == 0) {
-        umma::mma_chunk(tmem, htile, btile[0], mlp::kH, kRows, kChunkN, false);
+        umma::mma_chunk(tmem, htile, btile(0), mlp::kH, kRows, kChunkN, false);
         umma::mma_commit(&mbar_chunk[0]);
         last_mbar = &mbar_chunk[0];
         last_parity = 0;
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
             umma::fence_after_sync();
             if (!ok) break;
             if (tid == 0) {
-                umma::mma_chunk(tmem + (uint32_t)(((c + 1) & 1) * kChunkN), htile, btile[(c + 1) & 1], mlp::kH, kRows,
+                umma::mma_chunk(tmem + (uint32_t)(((c + 1) & 1) * kChunkN), htile, btile((c + 1) & 1), mlp::kH, kRows,
                                 kChunkN, false);
                 umma::mma_commit(&mbar_chunk[(c + 1) & 1]);
                 last_mbar = &mbar_chunk[(c + 1) & 1];
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
         ok_warp = ok_warp && w;
         if (w) {
         if (c + 2 < nch) {
-            copy_bytes(btile[c & 1], w4img + (size_t)(c + 2) * kChunkBytes, kChunkBytes);
+            copy_bytes(btile(c & 1), w4img + (size_t)(c + 2) * kChunkBytes, kChunkBytes);
             // chunk c - 1's biases, the third place, were last read before this chunk's barrier
             copy_bytes(b4s + (slot == 0 ? 2 : slot - 1) * kB4Bytes, b4img + (size_t)(c + 2) * kB4Bytes, kB4Bytes);
             cp_async_commit();
