@@ -15,7 +15,8 @@
 // both passes: 7.38 ms before these, 7.01 with the uniforms, 6.82 with the
 // biases, 6.72 with the rest; 6.28 once no tile's address was read from a
 // pointer array in local memory (a load from L2 a chunk), 5.78 with tile copies
-// of fixed size.  Two epilogues:
+// of fixed size, 5.67 with packed hidden-layer epilogues and a plain barrier a
+// chunk.  Two epilogues:
 //   kLse     log-sum-exp, arg-max and its probability per row;
 //   kSample  the learned-branch candidates: each row walks its softmax CDF
 //            once with its uniforms drawn as ascending order statistics; a
@@ -236,15 +237,15 @@ __device__ __forceinline__ void features(const mlp::ProposalDev &pd, const float
 
 // Writes 8 consecutive bf16 values (k = k0..k0+7) of row r into a K-major tile.
 __device__ __forceinline__ void put8(unsigned char *tile, int r, int k0, int K, const float *v) {
-    __align__(16) __nv_bfloat16 b[8];
+    __align__(16) __nv_bfloat162 b[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) b[i] = __float2bfloat16_rn(v[i]);
+    for (int i = 0; i < 4; ++i) b[i] = __float22bfloat162_rn(make_float2(v[2 * i], v[2 * i + 1]));
     *reinterpret_cast<uint4 *>(tile + umma::kmajor_offset(r, k0, K)) = *reinterpret_cast<const uint4 *>(b);
 }
 __device__ __forceinline__ void store8(__nv_bfloat16 *dst, const float *v) {
-    __align__(16) __nv_bfloat16 b[8];
+    __align__(16) __nv_bfloat162 b[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) b[i] = __float2bfloat16_rn(v[i]);
+    for (int i = 0; i < 4; ++i) b[i] = __float22bfloat162_rn(make_float2(v[2 * i], v[2 * i + 1]));
     *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(b);
 }
 
@@ -427,7 +428,15 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
             umma::tmem_ld32(lcol, warp, 0, *reinterpret_cast<float(*)[32]>(v));
             umma::tmem_ld32(lcol, warp, 32, *reinterpret_cast<float(*)[32]>(v + 32));
 #pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] = bf16r(fmaxf(v[j] + bias[64 * l + j], 0.0f));
+            for (int j = 0; j < 64; j += 4) {  // put8 rounds to bf16
+                const float4 b = *reinterpret_cast<const float4 *>(bias + 64 * l + j);
+                const float2 lo = __fadd2_rn(make_float2(v[j], v[j + 1]), make_float2(b.x, b.y)),
+                             hi = __fadd2_rn(make_float2(v[j + 2], v[j + 3]), make_float2(b.z, b.w));
+                v[j] = fmaxf(lo.x, 0.0f);
+                v[j + 1] = fmaxf(lo.y, 0.0f);
+                v[j + 2] = fmaxf(hi.x, 0.0f);
+                v[j + 3] = fmaxf(hi.y, 0.0f);
+            }
 #pragma unroll
             for (int j = 0; j < 64; j += 8) put8(htile, tid, j, mlp::kH, v + j);
             if (kMode == kLse && p.save) {  // as the tile itself: eight rows' 16 bytes are one 128-byte line
@@ -488,21 +497,19 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
         us[n_u * kRows] = INFINITY;
         next_u = us[0];
     }
-    // `ok` changes only at block barriers (uniform); `ok_warp` records this
-    // warp's waits and joins `ok` at the next barrier, so every warp passes
-    // the same sequence of barriers whatever fails.
-    bool ok_warp = true;
+    // Every warp passes the same barriers whatever fails: a warp whose wait ran
+    // out (ok_warp) does no more work and no more waits, thread 0 then issues no
+    // more products, and `ok` is settled after the chunks.
+    bool ok_warp = ok;
     int slot = 0;  // c % 3
-    for (int c = 0; c < nch; ++c, slot = slot == 2 ? 0 : slot + 1) {
-        if (!ok) break;
+    for (int c = 0; ok && c < nch; ++c, slot = slot == 2 ? 0 : slot + 1) {
         if (c + 1 < nch) {
             cp_async_wait_all();
             umma::fence_proxy_async();
             umma::fence_before_sync();
-            ok = __syncthreads_and(ok_warp) != 0;
+            __syncthreads();
             umma::fence_after_sync();
-            if (!ok) break;
-            if (tid == 0) {
+            if (tid == 0 && ok_warp) {
                 umma::mma_chunk(tmem + (uint32_t)(((c + 1) & 1) * kChunkN), htile, btile((c + 1) & 1), mlp::kH, kRows,
                                 kChunkN, false);
                 umma::mma_commit(&mbar_chunk[(c + 1) & 1]);
@@ -510,9 +517,8 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
                 last_parity = (uint32_t)(((c + 1) >> 1) & 1);
             }
         }
-        const bool w = mma_wait(&mbar_chunk[c & 1], (uint32_t)((c >> 1) & 1));
-        ok_warp = ok_warp && w;
-        if (w) {
+        ok_warp = ok_warp && mma_wait(&mbar_chunk[c & 1], (uint32_t)((c >> 1) & 1));
+        if (ok_warp) {
         if (c + 2 < nch) {
             copy_tile<kChunkBytes>(btile(c & 1), w4img + (size_t)(c + 2) * kChunkBytes);
             // chunk c - 1's biases, the third place, were last read before this chunk's barrier
@@ -591,7 +597,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
                 cum = end;
             }
         }
-        }  // w
+        }  // ok_warp
         umma::fence_before_sync();
     }
     ok = __syncthreads_and(ok && ok_warp) != 0;
