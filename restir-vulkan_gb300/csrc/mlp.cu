@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
 // one barrier, after which both products are issued (its dh3 and the next z).
 // 65,536 rows and 4096 clusters are 512 CTAs: with two an SM (88 KB, two
 // barriers a chunk, the hidden layers run again, the one-hot tested at every
-// column) they took 0.315 ms in two rounds; now 0.154 ms in one.
+// column) they took 0.315 ms in two rounds; now 0.149 ms in one.
 constexpr int kGOffH = 0;                                  // h3 tile, 128 x 64 bf16
 constexpr int kGOffDz = kGOffH + kRows * mlp::kH * 2;      // dz tile, 128 x 64 (K-major over clusters)
 constexpr int kGOffB = kGOffDz + kRows * kChunkN * 2;      // W4^T chunk (cluster x hidden)
@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_grad(const GradParams p) {
 // in registers meanwhile.  h3 comes in the tile's own layout: rows of a plain
 // matrix cost 33 cycles of the load pipe per instruction, and their transposed
 // stores conflict.  65,536 rows x 4096 clusters: 0.289 ms with one h tile, two
-// barriers and plain rows; 0.248 with the second tile; 0.158 with the layout
+// barriers and plain rows; 0.248 with the second tile; 0.152 with the layout
 // and the biases in shared memory.  256 threads and two CTAs an SM: 0.20.
 // dst[0..3] += v[0..3], dst on a 16-byte boundary
 __device__ __forceinline__ void red_add4(float *dst, const float *v) {
