@@ -351,6 +351,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
     copy_tile<kWeightImgBytes>(smem + kOffW1, reinterpret_cast<const unsigned char *>(p.pd.w123img));
     copy_tile<kChunkBytes>(btile(0), w4img);
     unsigned char *b4s = smem + kOffB4;
+    const float b4_first = tid < min(nch, 2) * kChunkN ? __ldg(p.pd.b4e + tid) : 0.0f;  // placed once the x tile is free
     const unsigned char *b4img = reinterpret_cast<const unsigned char *>(p.pd.b4e);
     cp_async_commit();
     if (nch > 1) copy_tile<kChunkBytes>(btile(1), w4img + kChunkBytes);
@@ -423,7 +424,7 @@ __global__ void __launch_bounds__(128, 4) k_mlp_fused(const FusedParams p) {
         const bool w = mma_wait(&mbar_layer, (uint32_t)(l & 1));
         if (w) {
             // the first two chunks' biases; the barriers of this loop come before their use
-            if (l == 1 && tid < min(nch, 2) * kChunkN) reinterpret_cast<float *>(b4s)[tid] = __ldg(p.pd.b4e + tid);
+            if (l == 1 && tid < min(nch, 2) * kChunkN) reinterpret_cast<float *>(b4s)[tid] = b4_first;
             float v[64];
             umma::tmem_ld32(lcol, warp, 0, *reinterpret_cast<float(*)[32]>(v));
             umma::tmem_ld32(lcol, warp, 32, *reinterpret_cast<float(*)[32]>(v + 32));
