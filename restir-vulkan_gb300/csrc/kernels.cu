@@ -496,8 +496,9 @@ __device__ __forceinline__ ResV<R, MIS> ris(const DevScene &s, const Texel &t, f
 #ifndef RG_RIS_MIN_BLOCKS
 #define RG_RIS_MIN_BLOCKS 8
 #endif
-// Two samples per reservoir: 80 registers and fewer spills beat two more
-// blocks (641x359 with MIS: 1.27 ms a frame at 8 blocks, 1.21 at 6).
+// Two samples per reservoir, or one pixel a thread: 80 registers and fewer spills
+// beat two more blocks (641x359 with MIS: 1.27 ms a frame at 8 blocks, 1.21 at 6;
+// 256x256, one pixel a thread: 0.104 and 0.097, 440x350 0.181 and 0.177).
 #ifndef RG_RIS_MIN_BLOCKS2
 #define RG_RIS_MIN_BLOCKS2 6
 #endif
@@ -639,7 +640,8 @@ __device__ __forceinline__ void initial_temporal_tile(const InitialParams &p, in
 }
 
 template <int PPT, int R, bool MIS>
-__global__ void __launch_bounds__(128, R == 1 ? RG_RIS_MIN_BLOCKS : RG_RIS_MIN_BLOCKS2) k_initial_temporal(const InitialParams p) {
+__global__ void __launch_bounds__(128, R == 1 && PPT > 1 ? RG_RIS_MIN_BLOCKS : RG_RIS_MIN_BLOCKS2)
+    k_initial_temporal(const InitialParams p) {
     initial_temporal_tile<PPT, R, MIS>(p, blockIdx.x, blockIdx.y);
 }
 
