@@ -284,16 +284,18 @@ int rg_reservoir_bytes(rg_context *ctx);
 
 /* ---- device layout of the tree ----
  * No counterpart in the reference.  Shadow rays on the filtered slab test's
- * fast path (every direction component nonzero, finite, within 2^+-100, and
- * for RG_TREE_QUANT4 within 2^+-60 from an origin within 2^40; no NaN box) may
- * walk a copy of the reference's tree built at upload; the others always walk
- * the reference's own tree.  Results are unchanged: the
- * reference's slab test is monotone under box containment for those rays.
+ * fast path (every direction component nonzero, finite, within 2^+-100; no NaN
+ * box) may walk a copy of the reference's tree built at upload; the others
+ * always walk the reference's own tree, and so do, for RG_TREE_QUANT4, those
+ * with a component below 2^-120 (|origin| + r), r the copy's reach, at most
+ * about 2^10 times the scene's extent plus its distance from 0.  Results are
+ * unchanged: the reference's slab test is monotone under box containment for
+ * those rays.
  *   RG_TREE_QUANT4 (the default): collapsed to four children per node, child
  *     boxes stored as 8-bit offsets decoding to boxes that contain the exact
  *     ones (64-byte nodes), each reached triangle tested with its exact box
  *     first.  Built when every child box of the tree lies inside the box its
- *     parent stores for it and every coordinate is finite and within 2^40.
+ *     parent stores for it and every box is finite (and below about 2^110).
  *     Measured fastest (1080p, 1.05M triangles: 2.8 ms per unbiased spatial
  *     pass).
  *   RG_TREE_WIDE4: the same collapse with exact boxes (128-byte nodes; each

@@ -650,10 +650,10 @@ int32_t host_pack_quant(const rg_aabb_tree_node *src, int32_t n, const float *tr
 // c + (2^15 + q) s, the scale of z with the slot masks in its low bits, inner
 // children in the first slots, a node's inner children consecutive (each
 // child's own children follow its group, first child first) and its leaf
-// records too, so a node holds two links.  Empty when a base or scale is
-// beyond 2^40, where the walk's products might overflow.
-std::vector<uint32_t> host_walk_nodes(const std::vector<uint32_t> &nodes) {
-    const float lim = 1099511627776.0f;
+// records too, so a node holds two links.  The bases and offsets ((2^15 + q) s
+// < 2^16 s) are finite, as the packing's own (2^23 + q) s is.
+std::vector<uint32_t> host_walk_nodes(const std::vector<uint32_t> &nodes, float *reach) {
+    float far = 0.0f;
     std::vector<uint32_t> out(nodes.size());
     struct Item { uint32_t from, to; };
     std::vector<Item> todo{{0u, 0u}};
@@ -670,7 +670,7 @@ std::vector<uint32_t> host_walk_nodes(const std::vector<uint32_t> &nodes) {
             float base;
             memcpy(&base, &w[a], 4);
             const float c = walk_base(eb[a], base);
-            if (!(std::fabs(c) <= lim) || !(pow2f(eb[a]) <= lim)) return {};
+            far = std::max(far, std::max(std::fabs(c), 65536.0f * pow2f(eb[a])));
             memcpy(&d[a], &c, 4);
         }
         int slot_of[4], ni = 0, at = 0;  // packed slot of each slot here
@@ -690,6 +690,7 @@ std::vector<uint32_t> host_walk_nodes(const std::vector<uint32_t> &nodes) {
         for (int k = ni - 1; k >= 0; --k) todo.push_back({w[12 + slot_of[k]], used + (uint32_t)k});
         used += (uint32_t)ni;
     }
+    if (reach) *reach = far;
     return out;
 }
 

@@ -25,9 +25,9 @@ int32_t host_pack_wide(const rg_aabb_tree_node *src, int32_t n, std::vector<floa
 bool host_tree_nested(const rg_aabb_tree_node *src, int32_t n);
 int32_t host_pack_quant(const rg_aabb_tree_node *src, int32_t n, const float *tris12, std::vector<uint32_t> &nodes,
                         std::vector<float> &leaves, int *wide_depth);
-// Packed quantized nodes -> the nodes the device walks; empty when the scene
-// is too large for the walk's arithmetic.
-std::vector<uint32_t> host_walk_nodes(const std::vector<uint32_t> &nodes);
+// Packed quantized nodes -> the nodes the device walks; *reach (may be null)
+// receives the largest magnitude among its bases and plane offsets.
+std::vector<uint32_t> host_walk_nodes(const std::vector<uint32_t> &nodes, float *reach = nullptr);
 void srgb_lut_host(float *out256);
 int host_trace_gbuffer(const float *nodes16, int32_t n_nodes, const float *tris12, int32_t n_tris,
                        const rg_material *mats, int32_t n_mats, const rg_camera &cam, int32_t w, int32_t h,

@@ -75,9 +75,10 @@ struct DevScene {
     const WNode *wide;            // 4-wide copy, or null (containment failed, NaN boxes, too deep)
     int32_t n_wide;
     int32_t wide_stack;           // stack entries the 4-wide walk may need (3 per level)
-    const QNode *qnodes;          // quantized 4-wide copy, or null (not nested, NaN or huge boxes, too deep)
+    const QNode *qnodes;          // quantized 4-wide copy, or null (not nested, NaN or infinite boxes, too deep)
     const QLeaf *qleaves;
     int32_t n_qnodes;
+    float walk_reach;             // of qnodes: rgm::walk_fits
     const GTri *tris;
     int32_t n_tris;
     const AliasLight *alias;      // point-light scenes

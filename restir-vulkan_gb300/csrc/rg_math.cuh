@@ -263,6 +263,18 @@ RG_HD void shadow_segment(f3 p1, f3 p2, f3 &o, f3 &d) {
     o = p1 + off;
     d = dir - scale(2.0f, off);
 }
+// Whether a segment may take the quantized walk (trace_pool.cuh), whose planes
+// are products of 1/d with at most `reach` (host_walk_nodes) and with |o|: with
+// the smallest |d| at least 2^-120 of their sum every product and sum there is
+// below 2^122.  The rule is relative, so a scene at any scale has the same fast
+// segments: all those of the filtered test (components within 2^+-100) where
+// reach + |o| is at most 2^20, and where it is larger those whose smallest
+// component is at least 2^-120 of it.
+RG_HD bool walk_fits(float reach, f3 o, f3 d) {
+    const float far = reach + fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z));
+    const float small = fminf(fminf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
+    return small >= far * 7.52316384526264005e-37f;  // 2^-120
+}
 
 // ---------------------------------------------------------------- G-buffer decoding
 RG_HD float half_bits_to_float(uint16_t h) {

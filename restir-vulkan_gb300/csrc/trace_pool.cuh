@@ -559,9 +559,8 @@ __device__ __forceinline__ uint4 as_uint4(float4 v) {
 // sides matter: a child is kept when
 //   max(0, near t's) < min(1, far t's),
 // which a reference hit (entry < 1, exit > 0, exit >= entry) implies.  The
-// clamps are the saturating form of the x axis' FMAs.  Magnitudes stay finite:
-// bases and scales are at most 2^40 (checked at upload), and the rays that
-// take this walk have |o| <= 2^40 and |d| in [2^-60, 2^60] (ray_fits); A or a
+// clamps are the saturating form of the x axis' FMAs.  Magnitudes stay finite
+// (rgm::walk_fits; the others walk the reference's tree exactly), and A or a
 // product that underflows is far below K.
 // Each axis' near and far code words are picked by the ray's direction sign.
 // One FMA a plane in place of decoding, subtracting o and multiplying by inv
@@ -604,15 +603,6 @@ __device__ __forceinline__ unsigned qlive(f3 o, f3 inv, const float4 &base, cons
         live = __funnelshift_l(__float_as_uint(max3f(tnx, ty.x, tz.x) - min3f(tfx, ty.y, tz.y)), live, 1);
     }
     return live;
-}
-// Whether the ray may take the quantized walk (finite products above); the
-// others walk the reference's tree exactly.
-__device__ __forceinline__ bool ray_fits(f3 o, f3 d) {
-    constexpr float kLo = 8.67361737988403547e-19f, kHi = 1.152921504606846976e18f;  // 2^-60, 2^60
-    constexpr float kPos = 1099511627776.0f;                                         // 2^40
-    const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
-    return fminf(fminf(ax, ay), az) >= kLo && max3f(ax, ay, az) <= kHi &&
-           max3f(fabsf(o.x), fabsf(o.y), fabsf(o.z)) <= kPos;
 }
 
 // The exact slab test of a leaf record's box (undecided filtered tests only).
@@ -715,7 +705,7 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
                     ++ts.skipped;
                 } else {
                     rgm::shadow_segment(p1, endpoint(owner), o, d);
-                    if (ray_inverse(d, inv) && ray_fits(o, d)) {
+                    if (ray_inverse(d, inv) && rgm::walk_fits(s.walk_reach, o, d)) {
                         busy = true;
                         gbase = 0u;
                         gmask = 1u;  // the root
