@@ -462,9 +462,9 @@ int32_t host_pack_wide(const rg_aabb_tree_node *src, int32_t n, std::vector<floa
 // upper code the smallest with D(q) >= its upper bound, so the decoded box
 // contains the child's box; every code also bounds its box as the device's
 // walk places planes (host_walk_nodes), with 1/16 code to spare, for which c
-// may lie a step lower and e one higher.  Leaf slots link (as ~index) to leaf records that hold the
-// triangle's exact box from the reference's tree and the triangle itself
-// (host_pack_tris form).
+// may lie a step lower and e one higher.  Inner children take the first slots.
+// Leaf slots link (as ~index) to leaf records that hold the triangle's exact
+// box from the reference's tree and the triangle itself (host_pack_tris form).
 //
 // The walk tests the decoded boxes only for a sure miss (a decoded box
 // contains the exact one, and the slab test is monotone under containment),
@@ -486,9 +486,6 @@ inline float pow2f(int eb) {
     memcpy(&s, &bits, 4);
     return s;
 }
-// D(q) for biased exponent eb and base c
-inline float qdecode(int q, int eb, float c) { return fmaf(8388608.0f + (float)q, pow2f(eb), c); }
-
 // The neighbouring floats of a finite x.
 inline float next_down(float x) {
     uint32_t u;
@@ -507,44 +504,70 @@ inline float walk_base(int eb, float base) {
     while ((double)c > v) c = next_down(c);
     return c;
 }
-inline double walk_plane(int q, int eb, float c) { return (double)c + (32768.0 + q) * (double)pow2f(eb); }
 
-// Code q bounds lo from below (hi from above): decoded, and as the walk's
-// plane with 1/16 code to spare (see trace_pool.cuh for what that covers).
-inline bool code_below(int q, int eb, float base, float c, float lo) {
-    return qdecode(q, eb, base) <= lo && walk_plane(q, eb, c) <= (double)lo - 0.0625 * (double)pow2f(eb);
-}
-inline bool code_above(int q, int eb, float base, float c, float hi) {
-    return qdecode(q, eb, base) >= hi && walk_plane(q, eb, c) >= (double)hi + 0.0625 * (double)pow2f(eb);
-}
+// One axis of a node: its biased exponent, the packed base and the walk's.
+struct QuantAxis {
+    int eb = 1;
+    float s = 0.0f, base = 0.0f, c = 0.0f;
+    double step = 0.0, inv_step = 0.0, pad = 0.0;  // s, 1 / s (exact), s / 16
 
-// Base and biased exponent of one axis of a node with bounds [lo, hi]; false
-// when no exponent up to 246 (255 * s finite) reaches hi.  A flat axis starts
-// at the exponent whose 255 codes span one unit in the last place of lo.
-bool quant_axis(float lo, float hi, float &c, int &eb) {
-    const double ext = (double)hi - (double)lo;
-    eb = 1;
-    if (ext > 0.0) eb = std::max(1, std::min(246, (int)std::ceil(std::log2(ext / 254.0)) + 127));
-    int lo_exp = 0;
-    std::frexp(std::max(std::fabs(lo), std::fabs(hi)), &lo_exp);
-    eb = std::max(eb, std::min(246, lo_exp - 1 - 23 - 8 + 127));
-    for (; eb <= 246; ++eb) {
-        const float s = pow2f(eb);
-        float cc = (float)((double)lo - 8388608.0 * (double)s);
-        if (!std::isfinite(cc)) continue;
-        while (fmaf(8388608.0f, s, cc) > lo) cc = next_down(cc);
-        while (fmaf(8388608.0f, s, next_up(cc)) <= lo) cc = next_up(cc);
-        if (!std::isfinite(qdecode(255, eb, cc))) continue;
-        // a step lower where the walk's plane of code 0 needs it
-        for (int k = 0; k < 2 && !code_below(0, eb, cc, walk_base(eb, cc), lo); ++k) cc = next_down(cc);
-        const float w = walk_base(eb, cc);
-        if (code_below(0, eb, cc, w, lo) && code_above(255, eb, cc, w, hi)) {
-            c = cc;
-            return true;
-        }
+    float decode(int q) const { return fmaf(8388608.0f + (float)q, s, base); }  // D(q)
+    double plane(int q) const { return (double)c + (32768.0 + q) * step; }
+    // Code q bounds lo from below (hi from above): decoded, and as the walk's
+    // plane with 1/16 code to spare (see trace_pool.cuh for what that covers).
+    bool below(int q, float lo) const { return decode(q) <= lo && plane(q) <= (double)lo - pad; }
+    bool above(int q, float hi) const { return decode(q) >= hi && plane(q) >= (double)hi + pad; }
+
+    void set_base(float b) {
+        base = b;
+        c = walk_base(eb, b);
     }
-    return false;
-}
+    // The axis of a node with bounds [lo, hi]; false when no exponent up to 246
+    // (255 * s finite) reaches hi.  A flat axis starts at the exponent whose 255
+    // codes span one unit in the last place of lo.
+    bool fit(float lo, float hi) {
+        const double ext = (double)hi - (double)lo;
+        int first = 1, e = 0;
+        if (ext > 0.0) {  // the first power of two that is at least ext / 254
+            const double m = std::frexp(ext / 254.0, &e);
+            first = std::max(1, std::min(246, e - (m == 0.5) + 127));
+        }
+        std::frexp(std::max(std::fabs(lo), std::fabs(hi)), &e);
+        first = std::max(first, std::min(246, e - 1 - 23 - 8 + 127));
+        for (eb = first; eb <= 246; ++eb) {
+            s = pow2f(eb);
+            step = (double)s;
+            inv_step = 1.0 / step;
+            pad = 0.0625 * step;
+            float b = (float)((double)lo - 8388608.0 * step);
+            if (!std::isfinite(b)) continue;
+            while (fmaf(8388608.0f, s, b) > lo) b = next_down(b);
+            while (fmaf(8388608.0f, s, next_up(b)) <= lo) b = next_up(b);
+            set_base(b);
+            if (!std::isfinite(decode(255))) continue;
+            // a step lower where the walk's plane of code 0 needs it
+            for (int k = 0; k < 2 && !below(0, lo); ++k) set_base(next_down(base));
+            if (below(0, lo) && above(255, hi)) return true;
+        }
+        return false;
+    }
+    // The largest code below lo and the smallest above hi (from the real-valued
+    // estimate, stepped to the exact code), or -1.
+    int lower(float lo) const {
+        const double est = std::floor(((double)lo - ((double)base + 8388608.0 * step)) * inv_step);
+        int q = (int)std::max(0.0, std::min(255.0, est));
+        while (q > 0 && !below(q, lo)) --q;
+        while (q < 255 && below(q + 1, lo)) ++q;
+        return q > 0 || below(0, lo) ? q : -1;
+    }
+    int upper(float hi) const {
+        const double est = std::ceil(((double)hi - ((double)base + 8388608.0 * step)) * inv_step);
+        int q = (int)std::max(0.0, std::min(255.0, est));
+        while (q < 255 && !above(q, hi)) ++q;
+        while (q > 0 && above(q - 1, hi)) --q;
+        return q < 255 || above(255, hi) ? q : -1;
+    }
+};
 
 struct QuantBuilder {
     const rg_aabb_tree_node *src;
@@ -556,39 +579,31 @@ struct QuantBuilder {
 
     int32_t build(int32_t x, int depth) {
         max_depth = std::max(max_depth, depth);
-        WEntry e[4];
-        const int n = expand4(src, x, e, ok);
+        WEntry given[4], e[4];
+        const int n = expand4(src, x, given, ok);
+        int ni = 0, nl = 0;
+        for (int k = 0; k < n; ++k) ni += given[k].ref >= 0;
+        for (int k = 0, at = 0; k < n; ++k) e[given[k].ref >= 0 ? at++ : ni + nl++] = given[k];
         const int32_t me = (int32_t)(nodes->size() / 16);
         nodes->resize(nodes->size() + 16, 0u);
         uint32_t w[16] = {0};
-        float base[3] = {0.0f, 0.0f, 0.0f};
-        int eb[3] = {1, 1, 1};
+        QuantAxis ax[3];
         for (int a = 0; a < 3; ++a) {
             float lo = e[0].lo[a], hi = e[0].hi[a];
             for (int k = 1; k < n; ++k) { lo = std::min(lo, e[k].lo[a]); hi = std::max(hi, e[k].hi[a]); }
-            if (!std::isfinite(lo) || !std::isfinite(hi) || !quant_axis(lo, hi, base[a], eb[a])) ok = false;
-            memcpy(&w[a], &base[a], 4);
+            if (!std::isfinite(lo) || !std::isfinite(hi) || !ax[a].fit(lo, hi)) ok = false;
+            memcpy(&w[a], &ax[a].base, 4);
         }
-        uint32_t leafbits = 0, innerbits = 0;
-        for (int k = 0; k < n; ++k) (e[k].ref < 0 ? leafbits : innerbits) |= 1u << k;
-        w[3] = (uint32_t)eb[0] | ((uint32_t)eb[1] << 8) | ((uint32_t)eb[2] << 16) | ((leafbits | innerbits << 4) << 24);
-        w[10] = (uint32_t)eb[0] << 23;  // s of x and y as floats (the walk reads them directly)
-        w[11] = (uint32_t)eb[1] << 23;
-        float wbase[3];
-        for (int a = 0; a < 3; ++a) wbase[a] = walk_base(eb[a], base[a]);
+        const uint32_t innerbits = (1u << ni) - 1u, leafbits = ((1u << n) - 1u) ^ innerbits;
+        w[3] = (uint32_t)ax[0].eb | ((uint32_t)ax[1].eb << 8) | ((uint32_t)ax[2].eb << 16) |
+               ((leafbits | innerbits << 4) << 24);
+        w[10] = (uint32_t)ax[0].eb << 23;  // s of x and y as floats (the walk reads them directly)
+        w[11] = (uint32_t)ax[1].eb << 23;
         for (int k = 0; k < 4 && ok; ++k) {
             const WEntry &c = e[k < n ? k : n - 1];  // an empty slot repeats the last child (ignored)
             for (int a = 0; a < 3; ++a) {
-                // start from the real-valued estimate, then step to the exact codes
-                const double s = (double)pow2f(eb[a]), o = (double)base[a] + 8388608.0 * s;
-                const float wb = wbase[a];
-                int ql = (int)std::max(0.0, std::min(255.0, std::floor(((double)c.lo[a] - o) / s)));
-                int qh = (int)std::max(0.0, std::min(255.0, std::ceil(((double)c.hi[a] - o) / s)));
-                while (ql > 0 && !code_below(ql, eb[a], base[a], wb, c.lo[a])) --ql;
-                while (ql < 255 && code_below(ql + 1, eb[a], base[a], wb, c.lo[a])) ++ql;
-                while (qh < 255 && !code_above(qh, eb[a], base[a], wb, c.hi[a])) ++qh;
-                while (qh > 0 && code_above(qh - 1, eb[a], base[a], wb, c.hi[a])) --qh;
-                if (!code_below(ql, eb[a], base[a], wb, c.lo[a]) || !code_above(qh, eb[a], base[a], wb, c.hi[a])) ok = false;
+                const int ql = ax[a].lower(c.lo[a]), qh = ax[a].upper(c.hi[a]);
+                if (ql < 0 || qh < 0) ok = false;
                 w[4 + 2 * a] |= (uint32_t)ql << (8 * k);
                 w[5 + 2 * a] |= (uint32_t)qh << (8 * k);
             }
@@ -673,22 +688,13 @@ std::vector<uint32_t> host_walk_nodes(const std::vector<uint32_t> &nodes, float 
             far = std::max(far, std::max(std::fabs(c), 65536.0f * pow2f(eb[a])));
             memcpy(&d[a], &c, 4);
         }
-        int slot_of[4], ni = 0, at = 0;  // packed slot of each slot here
-        for (int k = 0; k < 4; ++k)
-            if (inner >> k & 1u) slot_of[at++] = k;
-        ni = at;
-        for (int k = 0; k < 4; ++k)
-            if (leaf >> k & 1u) slot_of[at++] = k;
-        const uint32_t n_leaf = (uint32_t)(at - ni);
-        d[3] = ((uint32_t)eb[2] << 23) | (((1u << n_leaf) - 1u) << ni) | (((1u << ni) - 1u) << 4);
-        for (int q = 4; q < 10; ++q)
-            for (int k = 0; k < 4; ++k) d[q] |= ((w[q] >> (8 * slot_of[k < at ? k : at - 1])) & 255u) << (8 * k);
-        d[10] = w[10];
-        d[11] = w[11];
+        const uint32_t ni = (uint32_t)__builtin_popcount(inner);
+        d[3] = ((uint32_t)eb[2] << 23) | leaf | inner << 4;
+        memcpy(d + 4, w + 4, 8 * sizeof(uint32_t));  // codes, s of x and y
         d[12] = used;
-        d[13] = n_leaf ? ~w[12 + slot_of[ni]] - (uint32_t)ni : 0u;  // its leaves were packed together
-        for (int k = ni - 1; k >= 0; --k) todo.push_back({w[12 + slot_of[k]], used + (uint32_t)k});
-        used += (uint32_t)ni;
+        d[13] = leaf ? ~w[12 + ni] - ni : 0u;  // its leaves were packed together
+        for (uint32_t k = ni; k-- > 0;) todo.push_back({w[12 + k], used + k});
+        used += ni;
     }
     if (reach) *reach = far;
     return out;
