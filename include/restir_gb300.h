@@ -245,9 +245,11 @@ int rg_build_bvh(const float *tri_xyz, int32_t n_tris, rg_aabb_tree_node *out_no
  * returns the node count; *ref_undefined (host, may be null) is set when a
  * range took a path the reference leaves undefined (see rg_build_bvh).
  * At most 4,194,304 triangles; coordinates must be finite.  The context keeps
- * the workspace (about 170 bytes per triangle) for later calls until it is
- * destroyed.  No counterpart
- * in the reference, which builds on the host (aabbTreeBuilder.cpp:52-214). */
+ * the workspace for later calls until the next rg_upload_scene or rg_destroy:
+ * 183 bytes per triangle, and 4 bytes per tree level for every subtree of up to
+ * 128 triangles that a warp builds (2 to 3 bytes per triangle; more for a deep,
+ * uneven tree).  No counterpart in the reference, which builds on the host
+ * (aabbTreeBuilder.cpp:52-214). */
 int rg_build_bvh_device(rg_context *ctx, const float *tri_xyz, int32_t n_tris, rg_aabb_tree_node *nodes,
                         rg_triangle *triangles, int32_t *ref_undefined, void *stream);
 /* Depth of the tree (root = 1). */

@@ -108,7 +108,9 @@ struct rg_context {
     uint32_t vc_tag = 0;
     bool vc_on = true;        // rg_set_visibility_cache
     bool vc_dirty = true;     // clear before the next use (new scene, new buffers)
-    // workspace of rg_build_bvh_device (synchronous, so idle between calls)
+    // workspace of rg_build_bvh_device (synchronous, so idle between calls),
+    // given back by the next rg_upload_scene: a tree is built to be uploaded,
+    // and building every frame without an upload keeps it
     unsigned char *tree_ws[2] = {nullptr, nullptr};
     size_t tree_ws_bytes[2] = {0, 0};
 
@@ -118,6 +120,12 @@ struct rg_context {
         dev_free(nodes); dev_free(wide); dev_free(qnodes); dev_free(qleaves); dev_free(tris); dev_free(alias); dev_free(pl_color); dev_free(tri_lights);
         dev_free(tri_alias); dev_free(materials);
         has_scene = false;
+    }
+    void release_tree_workspace() {
+        for (int k = 0; k < 2; ++k) {
+            dev_free(tree_ws[k]);
+            tree_ws_bytes[k] = 0;
+        }
     }
     void release_frame() {
         dev_free(res[0]); dev_free(res[1]); dev_free(tmp); dev_free(image);
@@ -221,8 +229,7 @@ int rg_destroy(rg_context *ctx) {
     dev_free(ctx->mma_timeouts);
     dev_free(ctx->vc_buf[0]);
     dev_free(ctx->vc_buf[1]);
-    dev_free(ctx->tree_ws[0]);
-    dev_free(ctx->tree_ws[1]);
+    ctx->release_tree_workspace();
     delete ctx;
     return RG_OK;
 }
@@ -336,6 +343,7 @@ int rg_upload_scene(rg_context *ctx, const rg_scene_desc *sc) {
     if (sc->n_materials > 0 && !sc->materials) return fail(RG_ERR_INVALID_ARGUMENT, "null materials");
 
     ctx->release_scene();
+    ctx->release_tree_workspace();
     cudaError_t e = cudaSuccess;
     std::vector<float> n16(16 * (size_t)sc->n_nodes), t12(12 * (size_t)sc->n_triangles);
 #if RG_NODE_PREORDER

@@ -208,7 +208,8 @@ int rg_internal_check_spatial_args(const rg_gbuffer *g, const void *in, const vo
 void noalloc_forget_device(int device);
 
 // Device workspace of the tree builder (two slots), kept in the context and
-// grown when a call needs more; freed with the context.
+// grown when a call needs more; freed by the next scene upload or with the
+// context.
 int rg_internal_tree_workspace(rg_context *ctx, int slot, size_t bytes, void **out);
 
 // proposal.cu: the learned proposal attached to a context.
