@@ -1028,8 +1028,6 @@ __global__ void __launch_bounds__(128, RG_SHADE_MIN_BLOCKS) k_shade(const ShadeP
 
 // ---------------------------------------------------------------- visibility batch (testVisibility)
 // A block of T threads takes `chunk` segments into its pool and traces it.
-constexpr int kVisChunk = 512;
-
 template <int T>
 __global__ void __launch_bounds__(T, 1024 / T) k_visibility_batch(const DevScene s, const float4 *p1, const float4 *p2,
                                                                   uint8_t *out, int n, int chunk) {
@@ -1319,27 +1317,16 @@ cudaError_t launch_shade(const DevScene &s, const GBufView &g, const rg_reservoi
 cudaError_t launch_visibility_batch(const DevScene &s, const float4 *p1, const float4 *p2, uint8_t *out, int n,
                                     cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    auto launch = [&](auto kernel, int threads, int chunk) {
-        const size_t smem = (size_t)chunk * (sizeof(rgpool::Ray) + sizeof(float4)) +
-                            (size_t)threads * (size_t)(RG_STACK_LOCAL ? 0 : s.depth) * sizeof(int);
+    auto launch = [&](auto kernel, const VisLaunch &v) {
+        const size_t smem = (size_t)v.chunk * (sizeof(rgpool::Ray) + sizeof(float4)) +
+                            (size_t)v.threads * (size_t)(RG_STACK_LOCAL ? 0 : s.depth) * sizeof(int);
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kernel<<<(unsigned)((n + chunk - 1) / chunk), threads, smem, st>>>(s, p1, p2, out, n, chunk);
+        kernel<<<v.blocks, v.threads, smem, st>>>(s, p1, p2, out, n, v.chunk);
         return cudaGetLastError();
     };
-    // A batch of up to 32 segments a warp for 8 warps an SM goes out as single
-    // warps of 4 to 32 segments, so that it reaches every SM; a larger one as
-    // blocks of 128 to 512 segments.  Blocks of 512 at every size took 48 us
-    // for 512 segments, 50 us for 39,000 (780 triangles; 163 and 194 us with
-    // 1.05M); now 16 and 20 (45 and 86) us.  4, 8 or 16 warps an SM differ by
-    // 2 % up to 20,000 segments; 16 is 15 % slower at 39,000.
-    constexpr int kWarps = 152 * 8;
-    if (n <= kWarps * 32) {
-        const int per_warp = (n + kWarps - 1) / kWarps;
-        return launch(k_visibility_batch<32>, 32, per_warp < 4 ? 4 : per_warp);
-    }
-    const int per_block = (n + 152 * 8 - 1) / (152 * 8);
-    return launch(k_visibility_batch<128>, 128, per_block < 128 ? 128 : per_block < kVisChunk ? per_block : kVisChunk);
+    const VisLaunch v = vis_launch(n);
+    return v.threads == 32 ? launch(k_visibility_batch<32>, v) : launch(k_visibility_batch<128>, v);
 }
 
 // ---------------------------------------------------------------- views: parameter records and launches
