@@ -1,11 +1,13 @@
 // gbuffer_kernel.cu -- primary-ray G-buffer on the GPU (one thread per pixel,
-// closest hit on the uploaded tree).  Shares every operation with the host
-// tracer through rg_gbuffer.cuh, so both write identical planes.
+// closest hit on the uploaded tree).  Rays, triangle tests and shading are the
+// host tracer's (rg_gbuffer.cuh); the walk is a second version of
+// rgm::closest_hit with the same tests in the same order, so both write
+// identical planes (tests/test_gpu_launch_sizes.py, test_gpu_parity.py).
 //
 // Bound by instruction issue and the L1's data pipe (both 75 % busy; 18 of 32
-// lanes a warp at work).  1920x1080, 1.05M triangles: 1.28 ms with the node
-// read as single words, 1.02 ms with two 256-bit loads and 8 x 4 pixels a warp
-// (16 x 2: 1.05, 4 x 8: 1.03), 0.82 ms with the packed slab tests.
+// lanes a warp at work).  1920x1080, 1.05M triangles: 0.82 ms, against 1.02 ms
+// with scalar slab tests and 1.28 ms with the node read as single words too; 16 x
+// 2 or 4 x 8 pixels a warp are 1 to 3 % slower than 8 x 4.
 #include <cuda_runtime.h>
 
 #include "rg_gbuffer.cuh"

@@ -127,8 +127,8 @@ __device__ __forceinline__ ResV<R, MIS> load_resv(const rg_reservoir *base, size
     ResV<R, MIS> r;
     // the 64-byte format as two 256-bit loads where the buffer allows it (a
     // caller's need only be 16-byte aligned): a neighbour's reservoir is a
-    // gather, which costs the L1 per load, not per byte (1080p frame 12.32 ->
-    // 12.10 ms with the visibility cache's entries read so too)
+    // gather, which costs the L1 per load, not per byte (a 1080p frame 12.10 ms,
+    // 12.32 with 128-bit loads here and of the visibility cache's entries)
     if (L::kWords == 4 && (reinterpret_cast<uintptr_t>(base) & 31u) == 0u) {
         float4 c, m;
         rgpool::ldg256(p, r.pos_lum[0], r.nrm[0]);
@@ -319,16 +319,25 @@ __device__ __forceinline__ void count_block_rays(const DevScene &s, int rays, co
 #endif
 
 // Pixels per thread of the single-view launch (the batched one is tuned): 3
-// (32 x 12 tiles) for large frames, whose blocks then have enough segments to
-// keep their lanes at work to the end (1280x720: 1.36 ms for RIS, two biased
-// passes and shading, against 1.42 and 1.56 with 2 and 1); 1 while one-pixel
-// blocks all fit on the chip at once, where a thread's pixels one after the
+// (32 x 12 tiles; 2 with two samples a reservoir) for large frames, whose
+// blocks then have enough segments to keep their lanes at work to the end
+// (1280x720: 1.30 ms for RIS, two biased passes and shading, against 1.34 and
+// 1.55 with 2 and 1); 1 in small ones, where a thread's pixels one after the
 // other are the time (256x256, whole frame: 0.096 ms against 0.186).
+// The line is a measured one, not a residency limit: 6 one-pixel blocks of 128
+// an SM hold 116,736 pixels, and from there to 155,648 a second, partial round
+// runs.  RIS pass alone at 118,000 and 155,000 pixels, one against several
+// pixels a thread, soup of 100,000 / 780 cube / 1.05M rock triangles, us:
+//   one sample   239 : 289 and 275 : 306, 102 : 160 and 120 : 163, 233 : 312 and 267 : 320;
+//   two samples  338 : 340 and 406 : 366, 148 : 165 and 176 : 181, 332 : 348 and 398 : 365.
+// With one sample one pixel a thread stays ahead to about 230,000 pixels (332 :
+// 356, 140 : 181, 304 : 349; at 260,000 401 : 379 and 169 : 203), with two
+// either is ahead somewhere from 120,000 on, by at most 11 %.
 #ifndef RG_RIS_PPT
 #define RG_RIS_PPT 3
 #endif
 constexpr int kRisPpt = RG_RIS_PPT;
-constexpr uint64_t kRisSmallFrame = 152 * 8 * 128;  // pixels: 8 blocks of 128 on every SM
+constexpr uint64_t kRisSmallFrame = 155648;  // pixels
 
 struct InitialParams {
     DevScene s;
@@ -497,8 +506,8 @@ __device__ __forceinline__ ResV<R, MIS> ris(const DevScene &s, const Texel &t, f
 #define RG_RIS_MIN_BLOCKS 8
 #endif
 // Two samples per reservoir, or one pixel a thread: 80 registers and fewer spills
-// beat two more blocks (641x359 with MIS: 1.27 ms a frame at 8 blocks, 1.21 at 6;
-// 256x256, one pixel a thread: 0.104 and 0.097, 440x350 0.181 and 0.177).
+// beat two more blocks (641x359 with MIS: 1.157 ms a frame, 1.164 at 8; 256x256,
+// one pixel a thread: 0.095 and 0.103).
 #ifndef RG_RIS_MIN_BLOCKS2
 #define RG_RIS_MIN_BLOCKS2 6
 #endif
@@ -696,8 +705,9 @@ __device__ __forceinline__ void spatial_biased_tile(const SpatialParams &p, int 
     store_resv(p.out, i, r);
 }
 
-// 6 blocks per SM (80 registers, no spills): 256x256 frame 0.104 ms, against
-// 0.113 at 8; 5 and 4 blocks are 2 % slower at 1280x720.
+// 6 blocks per SM (80 registers, no spills): 256x256 frame 0.098 ms, against
+// 0.107 at 8, 1280x720 passes 1.306 against 1.327; 5 and 4 blocks are 2 % slower
+// at 1280x720.
 #ifndef RG_BIASED_MIN_BLOCKS
 #define RG_BIASED_MIN_BLOCKS 6
 #endif

@@ -11,12 +11,10 @@
 // slots and by the latency of the epilogues (55-60 % of the slots, 15 warps an
 // SM), so they read b4 from shared memory (global loads, even from L1, were
 // most of the stalls), and kSample draws a row's uniforms before its search
-// and kLse finds an arg-max by triples.  2,073,600 rows and 4096 clusters,
-// both passes: 7.38 ms before these, 7.01 with the uniforms, 6.82 with the
-// biases, 6.72 with the rest; 6.28 once no tile's address was read from a
-// pointer array in local memory (a load from L2 a chunk), 5.78 with tile copies
-// of fixed size, 5.67 with packed hidden-layer epilogues and a plain barrier a
-// chunk.  Two epilogues:
+// and kLse finds an arg-max by triples; tile addresses are arithmetic (a pointer
+// array would live in local memory, a load from L2 a chunk) and tile copies have
+// compile-time sizes.  2,073,600 rows and 4096 clusters, both passes: 5.66 ms,
+// 7.38 without these.  Two epilogues:
 //   kLse     log-sum-exp, arg-max and its probability per row;
 //   kSample  the learned-branch candidates: each row walks its softmax CDF
 //            once with its uniforms drawn as ascending order statistics; a
@@ -840,9 +838,9 @@ __global__ void __launch_bounds__(128, 4) k_mlp_grad(const GradParams p) {
 // product after the one barrier, from a second h tile, and that tile travels
 // in registers meanwhile.  h3 comes in the tile's own layout: rows of a plain
 // matrix cost 33 cycles of the load pipe per instruction, and their transposed
-// stores conflict.  65,536 rows x 4096 clusters: 0.289 ms with one h tile, two
-// barriers and plain rows; 0.248 with the second tile; 0.152 with the layout
-// and the biases in shared memory.  256 threads and two CTAs an SM: 0.20.
+// stores conflict.  65,536 rows x 4096 clusters: 0.152 ms; 0.289 with one h tile,
+// two barriers and plain rows, 0.20 with 256 threads and two CTAs an SM.
+
 // dst[0..3] += v[0..3], dst on a 16-byte boundary
 __device__ __forceinline__ void red_add4(float *dst, const float *v) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
