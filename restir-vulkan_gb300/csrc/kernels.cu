@@ -325,7 +325,7 @@ __device__ __forceinline__ void count_block_rays(const DevScene &s, int rays, co
 // 1.55 with 2 and 1); 1 in small ones, where a thread's pixels one after the
 // other are the time (256x256, whole frame: 0.096 ms against 0.186).
 // The line is a measured one, not a residency limit: 6 one-pixel blocks of 128
-// an SM hold 116,736 pixels, and from there to 155,648 a second, partial round
+// an SM hold 116,736 pixels, and from there to 155,648 a second, partial wave
 // runs.  RIS pass alone at 118,000 and 155,000 pixels, one against several
 // pixels a thread, soup of 100,000 / 780 cube / 1.05M rock triangles, us:
 //   one sample   239 : 289 and 275 : 306, 102 : 160 and 120 : 163, 233 : 312 and 267 : 320;
