@@ -696,6 +696,9 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
             if (idle) {
                 ts.visits += (unsigned)visits;  // the finished segment's node visits
                 visits = 0;
+                // loaded here, the segment's own loads cover it (batched views keep the
+                // scene in global memory: 0.5 % of a run where the test loads it)
+                const float reach = s.walk_reach;
                 const int k = atomicAdd(next, 1);
                 f3 p1;
                 if (k >= n) {
@@ -704,7 +707,7 @@ __device__ void trace_quant_loop(const DevScene &s, Fetch fetch, int n, int *nex
                     ++ts.skipped;
                 } else {
                     rgm::shadow_segment(p1, endpoint(owner), o, d);
-                    if (ray_inverse(d, inv) && rgm::walk_fits(s.walk_reach, o, d)) {
+                    if (ray_inverse(d, inv) && rgm::walk_fits(reach, o, d)) {
                         busy = true;
                         gbase = 0u;
                         gmask = 1u;  // the root
